@@ -38,3 +38,36 @@ def test_prod_rows(vectors, nodes, bs, arity, B, cuda_device):
         layer.backward(nf, ef)
         assert torch.equal(nf[bs:], spread + (1.0 if accumulate else 0.0))
         assert torch.all(nf[:bs] == 1.0)
+
+
+@pytest.mark.parametrize("bs,blocks,cats,B", [(1, 1, 2, 1), (2, 3, 5, 37), (4, 3, 256, 130), (8, 4, 257, 64), (16, 2, 64, 1023)])
+def test_input_values(bs, blocks, cats, B, cuda_device):
+    """Values, summed-out samples and the NaN of an impossible category, for variables whose
+    nodes straddle the kernel's groups of nodes."""
+    with juice.set_block_size(bs):
+        leaves = [juice.inputs(v, num_node_blocks=blocks, dist=Categorical(num_cats=cats)) for v in range(5)]
+    layer = juice.InputLayer(leaves, cum_nodes=bs, pc_num_vars=5).to(cuda_device)
+    gen = torch.Generator(device=cuda_device).manual_seed(B)
+    n = bs * blocks
+    theta = torch.rand([5, n, cats], generator=gen, device=cuda_device) + 0.01
+    with torch.no_grad():
+        layer.params.copy_(theta.reshape(-1))
+    data = torch.randint(0, cats, [5, B], generator=gen, device=cuda_device)
+    mask = torch.rand([B, 5], generator=gen, device=cuda_device) < 0.3
+    ref = theta.double().log().gather(2, data[:, None, :].expand(5, n, B))
+    nm = torch.full([bs + 5 * n, B], 3.0, device=cuda_device)
+    layer(data, nm)
+    # __logf: absolute error 2^-21.4 in [0.5, 2], 3 ulp of the result outside
+    assert torch.all((nm[bs:].double() - ref.reshape(-1, B)).abs() <= 4e-7 + 4e-7 * ref.reshape(-1, B).abs())
+    assert torch.all(nm[:bs] == 3.0)
+    full = nm.clone()
+    layer(data, nm, missing_mask=mask)
+    gone = mask.T[:, None, :].expand(5, n, B).reshape(-1, B)
+    assert torch.equal(nm[bs:], torch.where(gone, torch.zeros_like(full[bs:]), full[bs:]))
+    data[2, B // 2] = cats
+    layer(data, nm)
+    bad = torch.zeros([5, n, B], dtype=torch.bool, device=cuda_device)
+    bad[2, :, B // 2] = True
+    assert torch.equal(torch.isnan(nm[bs:]), bad.reshape(-1, B))
+    from pyjuice_b200 import _native as nat
+    assert nat.device_status(clear=True) == 4
