@@ -71,3 +71,40 @@ def test_input_values(bs, blocks, cats, B, cuda_device):
     assert torch.equal(torch.isnan(nm[bs:]), bad.reshape(-1, B))
     from pyjuice_b200 import _native as nat
     assert nat.device_status(clear=True) == 4
+
+
+@pytest.mark.parametrize("nodes,cats,B,missing", [(1, 2, 1, False), (16, 3, 513, True), (32, 64, 512, False),
+                                                  (48, 300, 1030, True), (96, 7000, 700, False)])
+def test_input_flows_and_em(nodes, cats, B, missing, cuda_device):
+    """Flow histogram (added to what the slots hold) and EM against FP64: one sample, more
+    samples than one chunk, fewer nodes than a tile, every node in one category, vocabularies
+    beyond a batch."""
+    with juice.set_block_size(1):
+        leaves = [juice.inputs(v, num_node_blocks=nodes, dist=Categorical(num_cats=cats)) for v in range(3)]
+    layer = juice.InputLayer(leaves, cum_nodes=1, pc_num_vars=3).to(cuda_device)
+    gen = torch.Generator(device=cuda_device).manual_seed(cats)
+    theta = torch.rand([3, nodes, cats], generator=gen, device=cuda_device) + 0.01
+    theta = theta / theta.sum(dim=2, keepdim=True)
+    data = torch.randint(0, cats, [3, B], generator=gen, device=cuda_device)
+    data[0] = cats - 1
+    mask = torch.rand([B, 3], generator=gen, device=cuda_device) < 0.4 if missing else None
+    nf = torch.rand([1 + 3 * nodes, B], generator=gen, device=cuda_device)
+    old = torch.rand([3, nodes, cats], generator=gen, device=cuda_device)
+    with torch.no_grad():
+        layer.params.copy_(theta.reshape(-1))
+    layer.init_param_flows(flows_memory=0.0)
+    layer.param_flows.copy_(old.reshape(-1))
+    layer.backward(data, nf, torch.zeros_like(nf), missing_mask=mask)
+    f = nf[1:].reshape(3, nodes, B).double()
+    gone = torch.zeros([3, nodes, B], dtype=torch.bool, device=cuda_device)
+    if missing:
+        gone = mask.T[:, None, :].expand(3, nodes, B)
+    ref = old.double().scatter_add(2, data[:, None, :].expand(3, nodes, B), torch.where(gone, 0.0, f))
+    ref += torch.where(gone, f, 0.0).sum(dim=2, keepdim=True) * theta.double()
+    got = layer.param_flows.reshape(3, nodes, cats).double()
+    # sums of at most B + 2 positive terms in FP32: relative error (B + 2) 2^-24
+    assert torch.all((got - ref).abs() <= (B + 2) * 2.0 ** -24 * ref)
+    layer.mini_batch_em(step_size=0.3, pseudocount=0.1)
+    new = 0.7 * theta.double() + 0.3 * (got + 0.1 / cats) / (got.sum(dim=2, keepdim=True) + 0.1)
+    # FP64 arithmetic rounded once to FP32
+    assert torch.all((layer.params.reshape(3, nodes, cats).double() - new).abs() <= 2.0 ** -23 * new)
