@@ -184,25 +184,38 @@ constexpr int kPackSplit = (128 * (KT / 8)) / 256;
 __device__ __forceinline__ void pack_tile_part(const float* __restrict__ params, const PcbLseTile& t, int rpb_log2,
                                                const int* __restrict__ kw, int w_stride, uint8_t* __restrict__ dst,
                                                int part) {
+    // Rows up to the next multiple of 32 (the accumulators of others are never used), all terms
+    // (zeros behind the tile's, which meet zero exponentials in the contractions).
     const int rpb_mask = (1 << rpb_log2) - 1;
     const int nk = min(t.k_cnt, KT);
-    {
-        const int c = part * 256 + threadIdx.x;
-        const int r = c % 128;
-        const int kg = c / 128;
-        float w[8];
-        const int64_t rb = (int64_t)t.w_add + (int64_t)(r >> rpb_log2) * t.g_stride + (int64_t)(r & rpb_mask) * w_stride;
+    const int c = part * 256 + threadIdx.x;
+    const int r = c % 128;
+    const int kg = c / 128;
+    if (r >= ((t.n_rows + 31) & ~31)) return;
+    float w[8];
+    const int64_t rb = (int64_t)t.w_add + (int64_t)(r >> rpb_log2) * t.g_stride + (int64_t)(r & rpb_mask) * w_stride;
+    const bool whole = r < t.n_rows && kg * 8 + 8 <= nk;
+    int o[8];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const int k = kg * 8 + j;
-            w[j] = (r < t.n_rows && k < nk) ? __ldg(params + (int64_t)__ldg(kw + t.k_off + k) + rb) : 0.f;
-        }
-        uint4 h, l;
-        split8(w, h, l);
-        const uint32_t off = (uint32_t)(r >> 3) * kSBO + (uint32_t)kg * kLBO + (uint32_t)(r & 7) * 16;
-        *reinterpret_cast<uint4*>(dst + off) = h;
-        *reinterpret_cast<uint4*>(dst + kHalfBytes + off) = l;
+    for (int j = 0; j < 8; ++j) o[j] = kg * 8 + j < nk ? __ldg(kw + t.k_off + kg * 8 + j) : 0;
+    // eight consecutive terms stored side by side (element-flow tables): two 16-byte loads
+    if (whole && w_stride >= 8 && o[7] == o[0] + 7 && o[1] == o[0] + 1 && o[2] == o[0] + 2 && o[3] == o[0] + 3 &&
+        o[4] == o[0] + 4 && o[5] == o[0] + 5 && o[6] == o[0] + 6 &&
+        ((reinterpret_cast<uintptr_t>(params) | ((uintptr_t)(o[0] + rb) * 4)) & 15) == 0) {
+        const float4 a = __ldg(reinterpret_cast<const float4*>(params + o[0] + rb));
+        const float4 b = __ldg(reinterpret_cast<const float4*>(params + o[0] + rb) + 1);
+        w[0] = a.x; w[1] = a.y; w[2] = a.z; w[3] = a.w;
+        w[4] = b.x; w[5] = b.y; w[6] = b.z; w[7] = b.w;
+    } else {
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+            w[j] = (r < t.n_rows && kg * 8 + j < nk) ? __ldg(params + (int64_t)o[j] + rb) : 0.f;
     }
+    uint4 h, l;
+    split8(w, h, l);
+    const uint32_t off = (uint32_t)(r >> 3) * kSBO + (uint32_t)kg * kLBO + (uint32_t)(r & 7) * 16;
+    *reinterpret_cast<uint4*>(dst + off) = h;
+    *reinterpret_cast<uint4*>(dst + kHalfBytes + off) = l;
 }
 
 // E4M3 packing of one tile by a CTA of 256 threads: thread (r, h) takes row r and terms
