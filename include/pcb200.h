@@ -434,6 +434,21 @@ int pcb_lse_contract_tc05_accum(const float* src, const float* src2, const float
                                 int32_t slices_per_cta, void* stream);
 
 /*
+ * pcb_lse_contract in its BF16 forms (prec 1: single operands, 2: split) for tiles of any
+ * number of terms, in one launch, with the samples along the tensor-memory lanes. `packed`
+ * holds the tiles' weights (pcb_pack_weights): of tile t itself (chunk_index NULL, tiles of
+ * at most 128 terms), or of its 128-term chunk j at packed + chunk_index[t * chunk_ld + j] *
+ * 65536 (chunk_ld: at least the chunks of every tile). `tile_rows`: at least the rows of
+ * every tile (<= 128). ksplit (1 .. 8): CTAs (a cluster) that share a tile's chunks. Rows of src, src2, aux and out need no alignment.
+ * Replaces the same reference kernels as pcb_lse_contract (sum_layer.py:454-568,
+ * 1572-1730).
+ */
+int pcb_lse_contract_tmem(const float* src, const float* src2, const float* aux, float* out, int64_t ld, int32_t B,
+                          const uint8_t* packed, const PcbLseTile* tiles, int32_t num_tiles, int32_t tile_rows,
+                          const int32_t* krow, const int32_t* chunk_index, int32_t chunk_ld, int32_t mode,
+                          int32_t prec, int32_t ksplit, void* stream);
+
+/*
  * Combine of long tiles contracted as chunks in one launch: every 128-term chunk j of the
  * tile holding output row dst_rows[r] wrote its partial result to row j * num_rows + r of
  * partials (pcb_lse_contract_tc05 on a table whose out_row fields point there);
@@ -508,6 +523,13 @@ int pcb_sum_par_generic(const float* node_flows, const float* node_mars, const f
  */
 int pcb_modify_flows(float* node_flows, const float* node_mars, int64_t ld, int32_t B,
                      int64_t row0, int64_t row1, void* stream);
+
+/*
+ * The same values written elsewhere: out row r - row0 = log(node_flows[r]) - node_mars[r] for
+ * rows row0 <= r < row1 (out has the same leading dimension; node_flows stays as it is).
+ */
+int pcb_flow_ratios(const float* node_flows, const float* node_mars, float* out, int64_t ld, int32_t B, int64_t row0,
+                    int64_t row1, void* stream);
 
 /*
  * Sum-layer parameter flows, contraction over the batch (see PcbPflowTile for the ids):

@@ -19,7 +19,7 @@ import torch
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "libpcb200.so")
 CSRC = os.path.join(_HERE, "csrc")
-SOURCES = ["capi_common.cu", "lse_contract.cu", "lse_contract_tc.cu", "lse_short.cu", "lse_tc05.cu", "prod_kernels.cu", "sum_pflows.cu",
+SOURCES = ["capi_common.cu", "lse_contract.cu", "lse_contract_tc.cu", "lse_short.cu", "lse_tc05.cu", "lse_tmem.cu", "prod_kernels.cu", "sum_pflows.cu",
            "sum_pflows_tc05.cu", "sum_generic.cu", "em_kernels.cu", "input_kernels.cu", "sample_kernels.cu", "sample_noalloc.cu",
            "input_soft.cu", "input_dists.cu", "input_poe.cu"]
 NVCC_FLAGS = ["-O3", "-std=c++17", "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-shared",
@@ -135,6 +135,8 @@ _SIGS = {
     "pcb_lse_contract_tc05_ws": ([c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int32, c_int64, c_int64, c_void_p,
                                   c_void_p, c_int32, c_void_p, c_int32, c_int32, c_int32, c_int32, c_int32, c_void_p],
                                  c_int32),
+    "pcb_lse_contract_tmem": ([c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int32, c_void_p, c_void_p, c_int32,
+                               c_int32, c_void_p, c_void_p, c_int32, c_int32, c_int32, c_int32, c_void_p], c_int32),
     "pcb_sum_fwd_generic": ([c_void_p, c_void_p, c_int64, c_int32, c_void_p, c_void_p, c_int32, c_int32, c_void_p,
                              c_void_p, c_int32, c_int32, c_float, c_void_p], c_int32),
     "pcb_sum_ele_generic": ([c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int32, c_void_p, c_void_p, c_int32,
@@ -143,6 +145,7 @@ _SIGS = {
     "pcb_sum_par_generic": ([c_void_p, c_void_p, c_void_p, c_int64, c_int32, c_void_p, c_void_p, c_void_p, c_int32,
                              c_int32, c_void_p, c_void_p, c_void_p, c_int32, c_int32, c_int32, c_void_p], c_int32),
     "pcb_modify_flows": ([c_void_p, c_void_p, c_int64, c_int32, c_int64, c_int64, c_void_p], c_int32),
+    "pcb_flow_ratios": ([c_void_p, c_void_p, c_void_p, c_int64, c_int32, c_int64, c_int64, c_void_p], c_int32),
     "pcb_sum_pflows": ([c_void_p, c_void_p, c_void_p, c_int64, c_int32, c_void_p, c_void_p, c_void_p, c_int32,
                         c_int32, c_void_p, c_void_p, c_void_p, c_int32, c_int32, c_int32, c_int32, c_void_p], c_int32),
     "pcb_sum_pflows_tc05": ([c_void_p, c_void_p, c_void_p, c_int64, c_int32, c_void_p, c_void_p, c_void_p, c_int32,

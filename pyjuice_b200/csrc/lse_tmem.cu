@@ -1,0 +1,1053 @@
+// Log-sum-exp contractions with the samples along the tensor-memory lanes, for tiles of any
+// number of terms (same result as pcb_lse_contract in its BF16 forms):
+//   acc[r, b] = sum_k W(k, r) * exp(src[krow[k], b] - m_b)
+// with mode 0 writing log(acc) + m (sum forward) and modes 1/2 writing acc * exp(aux + m)
+// (element flows; mode 2 first turns node flows into log f - log m).
+//
+// D[128 samples x n rows] = E[128 samples x k] W[k x n rows]: a thread owns one sample. It
+// reads its sample's values of the source rows (a warp reads whole 128-byte lines whatever the
+// alignment of the rows), keeps the maximum in a register, exponentiates, rounds to bf16 (hi
+// and, in the split form, the remainder's lo) and writes the A operand to tensor memory; the
+// packed weights are the B operand in shared memory, and the epilogue writes rows of 32
+// consecutive samples. So no operand passes through shared memory on its way to the tensor
+// cores, tiles of few rows cost only the columns they have, and the kernel is bound by the
+// rows it reads and writes and by the exponentials and logarithms (16 per SM and cycle).
+//
+// A CTA takes one tile and 128 samples: 8 warps (two per lane quarter, each with half of a
+// chunk's 128 terms) load, exponentiate and finish; warp 8 copies weights and row numbers
+// ahead and issues the MMAs. Two CTAs share an SM (256 tensor-memory columns each: 128
+// accumulators, 2 x 64 of A), so that one loads while the other computes.
+//
+// Tiles of more than 128 terms: the chunks are split over a cluster of up to 8 CTAs, which
+// exchange their accumulators through distributed shared memory and add them in rank order
+// (deterministic), each scaled from its CTA's maximum to the common one. A CTA with several
+// chunks starts D afresh for each and adds it to FP32 sums in shared memory: the tensor cores
+// truncate when they accumulate (about 3e-8 of the sum per instruction, always downwards), so
+// that 16 chunks accumulated in D would be 1.3e-5 too small, against 3e-7 this way.
+//
+// Measured (forward, split form, weights packed, graph-timed): 119 tiles of 128 x 128, batch 512
+// (70 MB): 19.2 us, 3.7 TB/s, against 35.8 us for the best of the forms that keep the samples in
+// shared memory (lse_tc05.cu); 200 regions of 256 x 256 (262 MB): 87.5 us, 3.0 TB/s, on the
+// persistent form below, against 370 us in 128-term chunks. What is left: a chunk costs about
+// 2,000 cycles of MMAs (three products), as many of exponentials, and its rows arrive at about
+// 20 bytes per SM and cycle.
+//
+// Every wait is bounded; a CTA whose wait runs out writes NaN rows and reports
+// PCB_STATUS_WAIT_TIMEOUT.
+#include <cooperative_groups.h>
+
+#include <algorithm>
+#include <type_traits>
+
+#include "tc05.cuh"
+
+namespace cg = cooperative_groups;
+
+namespace {
+
+using namespace pcb::tc05;
+
+constexpr int KT = 128;                        // terms per chunk
+constexpr int NS = 128;                        // samples per CTA (the MMA's M)
+constexpr int kComputeThreads = 256;
+constexpr int kThreads = kComputeThreads + 32;
+constexpr int HT = KT / 2;                     // terms per thread and chunk
+constexpr uint32_t kHalfBytes = 128 * KT * 2;  // one bf16 copy of a packed 128 x 128 tile
+constexpr uint32_t kTileBytes = 2 * kHalfBytes;
+constexpr uint32_t kLBO = 128;                 // bytes between core matrices along K
+constexpr uint32_t kSBO = (KT / 8) * 128;      // bytes between 8-row groups
+constexpr uint32_t kColsD = 128, kColsA = KT / 2, kCols = 256;
+constexpr int kMaxCluster = 8;
+
+struct Smem {
+    // the weights come first (n_pad x 128 x (hi + lo) bf16), and in their place, once the MMAs
+    // are done, what the cluster's other CTAs send: per CTA the column blocks owned here
+    uint32_t sum, part, max, rows, bar, slot, total;
+    __host__ __device__ Smem(int n_pad, bool several, int ks) {
+        const uint32_t w = (uint32_t)n_pad * KT * 4;
+        const int blocks = n_pad / 16, owned = (blocks + ks - 1) / ks;
+        const uint32_t recv = (uint32_t)((ks - 1) * owned) * 16 * NS * 4;
+        sum = w > recv ? w : recv;
+        part = sum + (several ? w : 0);  // [n_pad][NS] FP32 sums of a CTA with several chunks
+        max = part + 2 * 2 * NS * 4;       // [2 buffers][2 halves][NS] chunk maxima; [CTA][NS] final ones
+        rows = max + kMaxCluster * NS * 4; // [2 buffers][KT] source rows of a chunk
+        bar = rows + 2 * KT * 4;
+        slot = bar + 6 * 8;
+        total = slot + 16;
+    }
+};
+
+// D (tensor memory) += A (tensor memory, K-major) B (shared memory)
+__device__ __forceinline__ void mma_ts(uint32_t d, uint32_t a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}\n" ::"r"(d),
+        "r"(a), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+
+// 16 consecutive 32-bit columns of this thread's lane
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};\n" ::
+            "r"(taddr),
+        "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
+        "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+        : "memory");
+}
+
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&r)[8]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};\n" ::"r"(taddr), "r"(r[0]),
+                 "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+                 : "memory");
+}
+
+__device__ __forceinline__ void wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory"); }
+
+__device__ __forceinline__ void mbar_arrive(uint64_t* m) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(smem_u32(m)) : "memory");
+}
+
+__device__ __forceinline__ void mbar_expect_tx(uint64_t* m, uint32_t bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(smem_u32(m)), "r"(bytes) : "memory");
+}
+
+__device__ __forceinline__ void bulk_copy_g2s(void* dst, const void* src, uint32_t bytes, uint64_t* mbar) {
+    asm volatile(
+        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(
+            smem_u32(dst)),
+        "l"(src), "r"(bytes), "r"(smem_u32(mbar))
+        : "memory");
+}
+
+// Packed FP32 pairs (one instruction for two values)
+__device__ __forceinline__ uint64_t pair(float a, float b) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float2 unpair(uint64_t x) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(x));
+    return r;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("add.rn.ftz.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("mul.rn.ftz.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t r;
+    asm("fma.rn.ftz.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ float ex2(float x) {
+    float r;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+__device__ __forceinline__ float lg2(float x) {
+    float r;
+    asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+constexpr float kLog2e = 1.4426950408889634f, kLn2 = 0.6931471805599453f, kFloatMin = 1.17549435e-38f;
+
+// bf16 roundings of a pair (hi) and of what they leave (lo), packed
+__device__ __forceinline__ uint32_t bf16x2(float lo, float hi) {
+    uint32_t r;
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
+    return r;
+}
+
+// x[j] = log(x[j]) + m[j]: one logarithm and one multiply-add each while every x is a normal
+// number and every m finite (voted by the warp), else the careful form. SIGN -1 subtracts m.
+template <int N, int SIGN>
+__device__ __forceinline__ void log_add(float (&x)[N], const float (&m)[N]) {
+    float lo = x[0], ml = m[0];
+#pragma unroll
+    for (int j = 1; j < N; ++j) lo = fminf(lo, x[j]), ml = fminf(ml, m[j]);
+    if (__all_sync(0xffffffffu, lo >= kFloatMin && ml > -INFINITY)) {
+#pragma unroll
+        for (int j = 0; j < N; ++j) x[j] = fmaf(lg2(x[j]), kLn2, SIGN * m[j]);
+    } else {
+#pragma unroll
+        for (int j = 0; j < N; ++j) x[j] = m[j] == -INFINITY ? -INFINITY : pcb::fast_log(x[j]) + SIGN * m[j];
+    }
+}
+
+// 16 values down a column: to rows 0 .. rows - 1 of it, ld apart
+__device__ __forceinline__ void store16(float* __restrict__ dst, int64_t ld, const float (&x)[16], bool in, int rows) {
+    if (in && rows >= 16) {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) dst[(int64_t)j * ld] = x[j];
+    } else if (in) {
+#pragma unroll
+        for (int j = 0; j < 16; ++j)
+            if (j < rows) dst[(int64_t)j * ld] = x[j];
+    }
+}
+
+// Barrier of the 256 compute threads
+__device__ __forceinline__ void compute_sync() { asm volatile("bar.sync 1, 256;\n" ::: "memory"); }
+
+// Instruction descriptor: D f32, A and B bf16, both K-major, M = 128, N = n
+__device__ __forceinline__ uint32_t idesc_n(int n) {
+    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
+}
+
+// The MMAs of one chunk into a fresh accumulator d (a: A's hi columns, lo behind them; w, wl: the
+// weights' hi and lo). Tiles of several chunks take the small products first: what additions
+// to an already large accumulator truncate is then left by the hi * hi steps alone. Tiles of one
+// chunk take them step by step, like the other tcgen05 kernels, whose results theirs equal.
+template <bool SPLIT>
+__device__ __forceinline__ void issue_mmas(uint32_t d, uint32_t a, uint32_t w, uint32_t wl, int steps, uint32_t idesc,
+                                           bool small_first) {
+    if (!SPLIT || !small_first) {
+        for (int s = 0; s < steps; ++s) {
+            const uint32_t o = (uint32_t)s * 2 * kLBO;
+            mma_ts(d, a + s * 8, desc(w + o, kLBO, kSBO), idesc, s > 0 ? 1u : 0u);
+            if (SPLIT) {
+                mma_ts(d, a + s * 8, desc(wl + o, kLBO, kSBO), idesc, 1u);
+                mma_ts(d, a + kColsA + s * 8, desc(w + o, kLBO, kSBO), idesc, 1u);
+            }
+        }
+        return;
+    }
+    for (int s = 0; s < steps; ++s) {
+        const uint32_t o = (uint32_t)s * 2 * kLBO;
+        mma_ts(d, a + s * 8, desc(wl + o, kLBO, kSBO), idesc, s > 0 ? 1u : 0u);
+        mma_ts(d, a + kColsA + s * 8, desc(w + o, kLBO, kSBO), idesc, 1u);
+    }
+    for (int s = 0; s < steps; ++s) mma_ts(d, a + s * 8, desc(w + (uint32_t)s * 2 * kLBO, kLBO, kSBO), idesc, 1u);
+}
+
+template <int MODE, bool SPLIT>
+__global__ void __launch_bounds__(kThreads, 2)
+lse_tmem_kernel(const float* __restrict__ src, const float* __restrict__ src2, const float* __restrict__ aux,
+                float* __restrict__ out, int64_t ld, int B, const uint8_t* __restrict__ packed,
+                const PcbLseTile* __restrict__ tiles, const int* __restrict__ krow,
+                const int* __restrict__ chunk_index, int chunk_ld, int n_max, bool several,
+                int num_slices, int32_t* __restrict__ status) {
+    pcb::pdl_trigger();
+    extern __shared__ __align__(1024) uint8_t sm[];
+    cg::cluster_group cluster = cg::this_cluster();
+    const int ks = (int)cluster.num_blocks();
+    const int rank = (int)cluster.block_rank();
+    const Smem S(n_max, several, ks);
+    float* sSum = reinterpret_cast<float*>(sm + S.sum);  // [rows][samples]
+    float* sPart = reinterpret_cast<float*>(sm + S.part);
+    float* sMax = reinterpret_cast<float*>(sm + S.max);
+    int* sRows = reinterpret_cast<int*>(sm + S.rows);
+    uint64_t* barW = reinterpret_cast<uint64_t*>(sm + S.bar);  // weights of a chunk arrived
+    uint64_t* barM = barW + 1;                                 // MMAs of a chunk completed
+    uint64_t* barA = barW + 2;                                 // A operand of a chunk written
+    uint64_t* barR = barW + 3;                                 // [2] row numbers of a chunk written
+    uint32_t* slot = reinterpret_cast<uint32_t*>(sm + S.slot);
+
+    const int unit = blockIdx.x / ks;
+    const int tile_id = unit / num_slices;
+    const int b0 = (unit - tile_id * num_slices) * NS;
+    const PcbLseTile t = tiles[tile_id];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int n_pad = (t.n_rows + 15) & ~15;
+    const int nch_tile = (t.k_cnt + KT - 1) / KT;
+    const int nch = rank < nch_tile ? (nch_tile - rank + ks - 1) / ks : 0;  // chunks rank, rank + ks, ...
+    auto chunk_of = [&](int i) { return rank + i * ks; };
+    auto terms_of = [&](int i) { return min(KT, t.k_cnt - chunk_of(i) * KT); };
+
+    if (warp == 8) {
+        tmem_alloc(slot, kCols);
+        fence_before_sync();
+    }
+    if (tid == 0) {
+        mbar_init(barW, 1);
+        mbar_init(barM, 1);
+        mbar_init(barA, kComputeThreads / 32);
+        mbar_init(barR, 1);
+        mbar_init(barR + 1, 1);
+        slot[1] = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+    }
+    __syncthreads();
+    fence_after_sync();
+    const uint32_t taddr = slot[0];
+    bool fail = false;
+    float own[2][16];  // this thread's sums of the column blocks that its CTA owns
+
+    if (warp == 8) {
+        const int row0 = t.k_cnt > 0 ? __ldg(krow + t.k_off) : 0;
+        auto put_rows = [&](int i) {  // source rows of chunk i (compiled tables), the first one beyond its terms
+            const int nk = terms_of(i);
+            const int* kr = krow + t.k_off + chunk_of(i) * KT;
+            int* dst = sRows + (i & 1) * KT;
+#pragma unroll
+            for (int j = 0; j < KT / 32; ++j) {
+                const int k = lane + 32 * j;
+                dst[k] = k < nk ? __ldg(kr + k) : row0;
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(barR + (i & 1));
+        };
+        if (nch > 0) put_rows(0);
+        if (nch > 1) put_rows(1);
+        pcb::pdl_wait();
+        auto copy_weights = [&](int i) {
+            if (lane != 0) return;
+            const int c = chunk_index ? __ldg(chunk_index + (int64_t)tile_id * chunk_ld + chunk_of(i)) : tile_id;
+            const uint8_t* w = packed + (size_t)c * kTileBytes;
+            const uint32_t half = (uint32_t)n_pad * KT * 2;
+            mbar_expect_tx(barW, SPLIT ? 2 * half : half);
+            bulk_copy_g2s(sm, w, half, barW);
+            if (SPLIT) bulk_copy_g2s(sm + half, w + kHalfBytes, half, barW);
+        };
+        if (nch > 0) copy_weights(0);
+        for (int i = 0; i < nch; ++i) {
+            bool ok = mbar_wait_bounded(barA, (uint32_t)(i & 1));
+            ok = mbar_wait_bounded(barW, (uint32_t)(i & 1)) && ok;
+            fence_after_sync();
+            if (lane == 0) {
+                if (ok) {
+                    const uint32_t idesc = idesc_n(n_pad);
+                    const uint32_t w = smem_u32(sm), wl = w + (uint32_t)n_pad * KT * 2;
+                    const uint32_t a = taddr + kColsD;
+                    const int steps = (terms_of(i) + 15) / 16;
+                    issue_mmas<SPLIT>(taddr, a, w, wl, steps, idesc, nch_tile > 1);
+                } else {
+                    slot[1] = 1;
+                }
+                commit(barM);
+            }
+            __syncwarp();
+            if (i + 2 < nch) put_rows(i + 2);  // the compute warps have read the rows of chunk i
+            if (i + 1 < nch) {
+                if (!mbar_wait_bounded(barM, (uint32_t)(i & 1)) && lane == 0) slot[1] = 1;
+                copy_weights(i + 1);
+            }
+        }
+        if (ks > 1) {
+            asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
+            asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+        }
+    } else {
+        const int half = warp >> 2;
+        const int s = (warp & 3) * 32 + lane;  // this thread's sample (tensor-memory lane)
+        const uint32_t tlane = taddr + ((uint32_t)((warp & 3) * 32) << 16);
+        const bool active = b0 + (warp & 3) * 32 < B;  // any sample of this warp in the batch
+        const int b = min(b0 + s, B - 1);
+        const float* psrc = src + b;
+        const float* psrc2 = MODE == 2 ? src2 + b : nullptr;
+        float mref = -INFINITY, scale = 1.f;
+        pcb::pdl_wait();
+        const uint32_t traw = tlane + half * HT;                   // raw values, in D's columns
+        const uint32_t ta = tlane + kColsD + half * (HT / 2);      // hi, then lo
+        const uint64_t log2e = pair(kLog2e, kLog2e), minus1 = pair(-1.f, -1.f);
+        for (int i = 0; i < nch; ++i) {
+            if (!mbar_wait_bounded(barR + (i & 1), (uint32_t)((i >> 1) & 1))) fail = true;
+            const int4* rows = reinterpret_cast<const int4*>(sRows + (i & 1) * KT + half * HT);
+            const int nk = terms_of(i) - half * HT;  // terms of this half
+            if (i > 0) {
+                // the MMAs of the last chunk are done: A is free, and D goes to the sums
+                if (!mbar_wait_bounded(barM, (uint32_t)((i - 1) & 1))) fail = true;
+                fence_after_sync();
+#pragma unroll 1
+                for (int c = half * 16; c < n_pad; c += 32) {
+                    float d[16];
+                    tmem_ld16(tlane + c, d);
+                    wait_ld();
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) {
+                        float* p = sSum + (c + j) * NS + s;
+                        *p = (i > 1 ? *p * scale : 0.f) + d[j];
+                    }
+                }
+                fence_before_sync();
+                compute_sync();  // both halves have read D before either writes raw values to it
+                fence_after_sync();
+            }
+            // values of the source rows: their maximum, and themselves to tensor memory
+            float m = -INFINITY;
+            constexpr int G = MODE == 2 ? 16 : 32;  // rows in flight per thread (twice that in mode 2)
+#pragma unroll 1
+            for (int g = 0; g < HT; g += G) {
+                float v[G];
+                if (active && g < nk) {
+                    float m2[MODE == 2 ? G : 1];
+#pragma unroll
+                    for (int j = 0; j < G; j += 4) {
+                        const int4 r4 = rows[(g + j) / 4];
+                        const int rr[4] = {r4.x, r4.y, r4.z, r4.w};
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) {
+                            const int64_t o = (int64_t)rr[q] * ld;
+                            v[j + q] = __ldg(psrc + o);
+                            if (MODE == 2) m2[j + q] = __ldg(psrc2 + o);
+                        }
+                    }
+                    if constexpr (MODE == 2) log_add<G, -1>(v, m2);
+                    if (g + G > nk) {  // places beyond the chunk's terms count as -inf
+#pragma unroll
+                        for (int j = 0; j < G; ++j)
+                            if (g + j >= nk) v[j] = -INFINITY;
+                    }
+                } else {
+#pragma unroll
+                    for (int j = 0; j < G; ++j) v[j] = -INFINITY;
+                }
+#pragma unroll
+                for (int j = 0; j < G; j += 2) m = fmaxf(m, fmaxf(v[j], v[j + 1]));
+#pragma unroll
+                for (int j = 0; j < G; j += 16) {
+                    uint32_t w[16];
+#pragma unroll
+                    for (int q = 0; q < 16; ++q) w[q] = __float_as_uint(v[j + q]);
+                    tmem_st16(traw + g + j, w);
+                }
+            }
+            wait_st();
+            float* part = sPart + (i & 1) * 2 * NS;
+            part[half * NS + s] = m;
+            compute_sync();
+            m = fmaxf(fmaxf(m, part[(half ^ 1) * NS + s]), mref);
+            scale = m == mref ? 1.f : pcb::fast_exp(mref - m);  // of the sums so far
+            mref = m;
+            const float mu = mref == -INFINITY ? 0.f : mref;
+            const uint64_t nmu = pair(-mu, -mu);
+#pragma unroll 1
+            for (int g = 0; g < HT; g += 16) {
+                float v[16];
+                tmem_ld16(traw + g, v);
+                wait_ld();
+                uint32_t hi[8], lo[8];
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    const uint64_t x = mul2(add2(pair(v[2 * j], v[2 * j + 1]), nmu), log2e);
+                    const float2 x2 = unpair(x);
+                    const float e0 = ex2(x2.x), e1 = ex2(x2.y);
+                    hi[j] = bf16x2(e0, e1);
+                    if (SPLIT) {
+                        const uint64_t h = pair(__uint_as_float(hi[j] << 16), __uint_as_float(hi[j] & 0xffff0000u));
+                        const float2 l = unpair(fma2(h, minus1, pair(e0, e1)));
+                        lo[j] = bf16x2(l.x, l.y);
+                    }
+                }
+                tmem_st8(ta + g / 2, hi);
+                if (SPLIT) tmem_st8(ta + kColsA + g / 2, lo);
+            }
+            wait_st();
+            fence_before_sync();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(barA);
+        }
+        const bool in = b0 + s < B;
+        const int nb16 = n_pad / 16;  // column blocks, alternating between the halves
+        const bool none = mref == -INFINITY;  // no term above -inf: log 0 / no flow
+        const bool solo = ks == 1;
+        // element values of a column block, one block ahead of their use
+        float a[MODE == 0 ? 1 : 16];
+        auto load_aux = [&](int blk) {
+            if constexpr (MODE != 0) {
+                if (!active || blk >= nb16) return;
+                const float* ax = aux + ((int64_t)t.aux_row + blk * 16) * ld + b;
+#pragma unroll
+                for (int j = 0; j < 16; ++j) a[j] = __ldg(ax + (int64_t)min(j, t.n_rows - 1 - blk * 16) * ld);
+            }
+        };
+        if (solo) load_aux(half);
+        if (nch > 0 && !mbar_wait_bounded(barM, (uint32_t)((nch - 1) & 1))) fail = true;
+        fence_after_sync();
+        fail = fail || slot[1] != 0;
+        if (solo) {
+#pragma unroll 1
+            for (int blk = half; blk < nb16; blk += 2) {
+                float d[16];
+                tmem_ld16(tlane + blk * 16, d);
+                wait_ld();
+                if (nch > 1) {
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) d[j] += sSum[(blk * 16 + j) * NS + s] * scale;
+                }
+                // all values first, then all stores: 16 independent chains
+                if (MODE == 0) {
+                    float m[16];
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) m[j] = mref;
+                    log_add<16, 1>(d, m);
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) d[j] = none ? 0.f : d[j] * ex2((a[MODE == 0 ? 0 : j] + mref) * kLog2e);
+                    load_aux(blk + 2);
+                }
+                if (fail) {
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) d[j] = __int_as_float(0x7fc00000);
+                }
+                store16(out + ((int64_t)t.out_row + blk * 16) * ld + b0 + s, ld, d, in, t.n_rows - blk * 16);
+            }
+        } else {
+            // Column block c belongs to CTA c % ks. This thread's own blocks (its half takes every
+            // other one, two at most) to registers, the others to their owners once every CTA
+            // of the cluster is done with its weights.
+            asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
+            auto sums = [&](int blk, float (&d)[16]) {
+                if (nch > 0) {
+                    tmem_ld16(tlane + blk * 16, d);
+                    wait_ld();
+                }
+#pragma unroll
+                for (int j = 0; j < 16; ++j) {
+                    if (nch == 0) d[j] = 0.f;
+                    if (nch > 1) d[j] += sSum[(blk * 16 + j) * NS + s] * scale;
+                    if (fail) d[j] = __int_as_float(0x7fc00000);
+                }
+            };
+#pragma unroll
+            for (int o = 0; o < 2; ++o) {
+                const int blk = rank + ks * (half + 2 * o);
+                if (blk < nb16) sums(blk, own[o]);
+            }
+            asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+            const int owned_max = (nb16 + ks - 1) / ks;
+            for (int blk = half; blk < nb16; blk += 2) {
+                const int to = blk % ks;
+                if (to == rank) continue;
+                float d[16];
+                sums(blk, d);
+                const int from = rank < to ? rank : rank - 1;  // place among the owner's senders
+                float* dst = cluster.map_shared_rank(reinterpret_cast<float*>(sm), to) +
+                             (size_t)((from * owned_max + blk / ks) * 16) * NS + s;
+#pragma unroll
+                for (int j = 0; j < 16; ++j) dst[j * NS] = d[j];
+            }
+            if (half == 0) {
+                for (int r = 0; r < ks; ++r) cluster.map_shared_rank(sMax, r)[rank * NS + s] = mref;
+            }
+        }
+        fence_before_sync();
+    }
+    if (fail) pcb::report_status(status, PCB_STATUS_WAIT_TIMEOUT);
+    __syncthreads();
+    if (warp == 8) {
+        fence_after_sync();
+        tmem_dealloc(taddr, kCols);
+    }
+    if (ks == 1) return;
+    cluster.sync();
+    if (warp == 8) return;
+    const int half = warp >> 2;
+    const int s = (warp & 3) * 32 + lane;
+    const bool in = b0 + s < B;
+    // own sums + what the others sent, in rank order, each scaled to the common maximum
+    float f[kMaxCluster];
+    float mm = -INFINITY;
+#pragma unroll
+    for (int r = 0; r < kMaxCluster; ++r) {
+        f[r] = r < ks ? sMax[r * NS + s] : -INFINITY;
+        mm = fmaxf(mm, f[r]);
+    }
+#pragma unroll
+    for (int r = 0; r < kMaxCluster; ++r) f[r] = f[r] == -INFINITY ? 0.f : pcb::fast_exp(f[r] - mm);
+    const int nb16 = n_pad / 16;
+    const int owned_max = (nb16 + ks - 1) / ks;
+#pragma unroll
+    for (int o = 0; o < 2; ++o) {
+        const int blk = rank + ks * (half + 2 * o);
+        if (blk >= nb16) break;
+        float a[16], x[16];
+        if (MODE != 0) {
+            const float* ax = aux + ((int64_t)t.aux_row + blk * 16) * ld + b0 + s;
+#pragma unroll
+            for (int j = 0; j < 16; ++j) a[j] = in ? __ldg(ax + (int64_t)min(j, t.n_rows - 1 - blk * 16) * ld) : 0.f;
+        }
+#pragma unroll
+        for (int j = 0; j < 16; ++j) x[j] = 0.f;
+#pragma unroll
+        for (int r = 0; r < kMaxCluster; ++r) {
+            if (r >= ks) break;
+            if (r == rank) {
+#pragma unroll
+                for (int j = 0; j < 16; ++j) x[j] += own[o][j] * f[r];
+            } else {
+                const float* p = reinterpret_cast<const float*>(sm) +
+                                 (size_t)(((r < rank ? r : r - 1) * owned_max + half + 2 * o) * 16) * NS + s;
+#pragma unroll
+                for (int j = 0; j < 16; ++j) x[j] += p[j * NS] * f[r];
+            }
+        }
+        if (MODE == 0) {
+            float m[16];
+#pragma unroll
+            for (int j = 0; j < 16; ++j) m[j] = mm;
+            log_add<16, 1>(x, m);
+        } else {
+#pragma unroll
+            for (int j = 0; j < 16; ++j) x[j] = mm == -INFINITY ? 0.f : x[j] * ex2((a[j] + mm) * kLog2e);
+        }
+        store16(out + ((int64_t)t.out_row + blk * 16) * ld + b0 + s, ld, x, in, t.n_rows - blk * 16);
+    }
+}
+
+// ---------------------------------------------------------------------------------------
+// Persistent form, for layers with a (tile, 128-sample slice) unit per SM or more: one CTA per
+// SM walks a contiguous run of units, chunk by chunk (q = 0, 1, ... over all of them). 16
+// compute warps (four per lane quarter, 32 terms of a chunk each) hold a chunk's values in
+// registers; warp 16 issues the MMAs and copies weights and row numbers ahead. A, D and the
+// weights are double buffered (slot q & 1): while chunk q's MMAs run, the compute warps have
+// the rows of chunk q + 1 in flight, and finish the unit that ended at q - 1. A unit of two
+// chunks keeps both accumulators apart until its end; of more, the older one goes to FP32 sums
+// in shared memory (for the same reason as above). Consecutive slices of a tile reuse its
+// weights.
+constexpr int kPWarps = 16;
+constexpr int kPThreads = 32 * kPWarps + 32;
+constexpr int PT = KT / 4;  // terms per thread and chunk
+constexpr int EB = 8;       // accumulator columns per epilogue step
+constexpr int kRowRing = 4;
+
+struct PSmem {
+    uint32_t sum, part, rows, bar, slot, total;  // two weight slots come first
+    __host__ __device__ PSmem(int n_pad, bool sums) {
+        const uint32_t w = (uint32_t)n_pad * KT * 4;
+        sum = 2 * w;
+        part = sum + (sums ? w : 0);        // [2 buffers][4 parts][NS] chunk maxima
+        rows = part + 2 * 4 * NS * 4;       // [kRowRing][KT]
+        bar = rows + kRowRing * KT * 4;
+        slot = bar + 16 * 8;
+        total = slot + 16;
+    }
+};
+
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&v)[8]) {
+    uint32_t r[8];
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(taddr));
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
+}
+
+// exp(m - to) for a scale between maxima; equal ones (also both -inf) give 1
+__device__ __forceinline__ float rescale(float m, float to) { return m == to ? 1.f : pcb::fast_exp(m - to); }
+
+template <int MODE, bool SPLIT>
+__global__ void __launch_bounds__(kPThreads, 1)
+lse_tmem_persistent_kernel(const float* __restrict__ src, const float* __restrict__ src2,
+                           const float* __restrict__ aux, float* __restrict__ out, int64_t ld, int B,
+                           const uint8_t* __restrict__ packed, const PcbLseTile* __restrict__ tiles,
+                           const int* __restrict__ krow, const int* __restrict__ chunk_index, int chunk_ld, int n_max,
+                           bool sums, int num_slices, int num_units, int32_t* __restrict__ status) {
+    pcb::pdl_trigger();
+    extern __shared__ __align__(1024) uint8_t sm[];
+    const PSmem S(n_max, sums);
+    const uint32_t wslot = (uint32_t)n_max * KT * 4;
+    float* sSum = reinterpret_cast<float*>(sm + S.sum);  // [rows][samples]
+    float* sPart = reinterpret_cast<float*>(sm + S.part);
+    int* sRows = reinterpret_cast<int*>(sm + S.rows);
+    uint64_t* barW = reinterpret_cast<uint64_t*>(sm + S.bar);  // [2] weights arrived
+    uint64_t* barM = barW + 2;                                 // [2] MMAs completed
+    uint64_t* barA = barW + 4;                                 // [2] A written, D read
+    uint64_t* barR = barW + 6;                                 // [kRowRing] row numbers written
+    uint32_t* slot = reinterpret_cast<uint32_t*>(sm + S.slot);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int u0 = (int)((int64_t)num_units * blockIdx.x / gridDim.x);
+    const int u1 = (int)((int64_t)num_units * (blockIdx.x + 1) / gridDim.x);
+
+    if (warp == kPWarps) {
+        tmem_alloc(slot, 512);
+        fence_before_sync();
+    }
+    if (tid == 0) {
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(barW + i, 1);
+            mbar_init(barM + i, 1);
+            mbar_init(barA + i, kPWarps);
+        }
+        for (int i = 0; i < kRowRing; ++i) mbar_init(barR + i, 1);
+        slot[1] = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+    }
+    __syncthreads();
+    fence_after_sync();
+    const uint32_t taddr = slot[0];
+    // columns: D of slots 0 and 1, then A (hi, lo) of slots 0 and 1
+    auto d_cols = [&](int q) { return taddr + (q & 1) * kColsD; };
+    auto a_cols = [&](int q) { return taddr + 2 * kColsD + (q & 1) * 2 * kColsA; };
+    auto chunks_of = [&](const PcbLseTile& t) { return max(1, (t.k_cnt + KT - 1) / KT); };
+    bool fail = false;
+
+    if (warp == kPWarps) {
+        // position of the next chunk whose row numbers, and whose weights, are fetched
+        int ru = u0, ri = 0, rq = 0, wu = u0, wi = 0, wq = 0;
+        int held[2] = {-1, -1}, loads[2] = {0, 0};
+        auto put_rows = [&]() {
+            if (ru >= u1) return;
+            const PcbLseTile t = tiles[ru / num_slices];
+            int* dst = sRows + (rq % kRowRing) * KT;
+#pragma unroll
+            for (int j = 0; j < KT / 32; ++j) {
+                const int k = ri * KT + lane + 32 * j;
+                dst[lane + 32 * j] = t.k_cnt > 0 ? __ldg(krow + t.k_off + (k < t.k_cnt ? k : 0)) : 0;
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(barR + rq % kRowRing);
+            ++rq;
+            if (++ri == chunks_of(t)) ri = 0, ++ru;
+        };
+        auto copy_weights = [&]() {
+            if (wu >= u1) return;
+            const int tile_id = wu / num_slices;
+            const PcbLseTile t = tiles[tile_id];
+            const int c = chunk_index ? __ldg(chunk_index + (int64_t)tile_id * chunk_ld + wi) : tile_id;
+            const int sl = wq & 1;
+            if (held[sl] != c) {
+                held[sl] = c;
+                ++loads[sl];
+                if (lane == 0) {
+                    const uint8_t* w = packed + (size_t)c * kTileBytes;
+                    const uint32_t half = (uint32_t)((t.n_rows + 15) & ~15) * KT * 2;
+                    mbar_expect_tx(barW + sl, SPLIT ? 2 * half : half);
+                    bulk_copy_g2s(sm + sl * wslot, w, half, barW + sl);
+                    if (SPLIT) bulk_copy_g2s(sm + sl * wslot + half, w + kHalfBytes, half, barW + sl);
+                }
+            }
+            ++wq;
+            if (++wi == chunks_of(t)) wi = 0, ++wu;
+        };
+        put_rows();
+        put_rows();
+        put_rows();
+        pcb::pdl_wait();
+        copy_weights();
+        int q = 0;
+        for (int u = u0; u < u1; ++u) {
+            const PcbLseTile t = tiles[u / num_slices];
+            const int nch = chunks_of(t);
+            const int n_pad = (t.n_rows + 15) & ~15;
+            for (int i = 0; i < nch; ++i, ++q) {
+                const int sl = q & 1;
+                // chunk q + 1's weights once the MMAs of chunk q - 1 have left their slot
+                if (q > 0 && !mbar_wait_bounded(barM + (sl ^ 1), (uint32_t)(((q - 1) >> 1) & 1)) && lane == 0) slot[1] = 1;
+                copy_weights();
+                bool ok = mbar_wait_bounded(barA + sl, (uint32_t)((q >> 1) & 1));
+                ok = mbar_wait_bounded(barW + sl, (uint32_t)((loads[sl] - 1) & 1)) && ok;
+                fence_after_sync();
+                if (lane == 0) {
+                    if (ok) {
+                        const uint32_t idesc = idesc_n(n_pad);
+                        const uint32_t w = smem_u32(sm + sl * wslot), wl = w + (uint32_t)n_pad * KT * 2;
+                        const uint32_t a = a_cols(q), d = d_cols(q);
+                        const int steps = max(1, (min(KT, t.k_cnt - i * KT) + 15) / 16);
+                        issue_mmas<SPLIT>(d, a, w, wl, steps, idesc, nch > 1);
+                    } else {
+                        slot[1] = 1;
+                    }
+                    commit(barM + sl);
+                }
+                __syncwarp();
+                put_rows();  // chunk q + 3: the rows of chunk q - 1 have been read
+            }
+        }
+        // the copies in flight (at most one beyond the last MMA's) have all been waited for above
+    } else {
+        const int part = warp >> 2;
+        const int s = (warp & 3) * 32 + lane;  // this thread's tensor-memory lane
+        const uint32_t tlane = (uint32_t)((warp & 3) * 32) << 16;
+        const uint64_t log2e = pair(kLog2e, kLog2e), minus1 = pair(-1.f, -1.f);
+        pcb::pdl_wait();
+
+        constexpr int NL = MODE == 2 ? PT / 2 : PT;  // terms loaded ahead
+        float v[PT], w[MODE == 2 ? NL : 1];
+        // rows [j0, j0 + NL) of chunk q of a unit with first sample b0 into v (and w)
+        auto load = [&](int q, int b0, int k_cnt, auto first) {
+            constexpr int j0 = decltype(first)::value;
+            if (b0 + (warp & 3) * 32 >= B || k_cnt <= 0) return;
+            const int64_t b = min(b0 + s, B - 1);
+            const int4* rows = reinterpret_cast<const int4*>(sRows + (q % kRowRing) * KT + part * PT + j0);
+#pragma unroll
+            for (int j = 0; j < NL; j += 4) {
+                const int4 r4 = rows[j / 4];
+                const int rr[4] = {r4.x, r4.y, r4.z, r4.w};
+#pragma unroll
+                for (int z = 0; z < 4; ++z) {
+                    const int64_t o = (int64_t)rr[z] * ld + b;
+                    v[j0 + j + z] = __ldg(src + o);
+                    if (MODE == 2) w[MODE == 2 ? j + z : 0] = __ldg(src2 + o);
+                }
+            }
+        };
+        auto wait_rows = [&](int q) {
+            if (!mbar_wait_bounded(barR + q % kRowRing, (uint32_t)((q / kRowRing) & 1))) fail = true;
+        };
+        // log f - log m of the terms loaded last (mode 2)
+        auto to_log = [&](auto first) {
+            constexpr int j0 = decltype(first)::value;
+            if constexpr (MODE == 2) {
+                float f[NL];
+#pragma unroll
+                for (int j = 0; j < NL; ++j) f[j] = v[j0 + j];
+                log_add<NL, -1>(f, w);
+#pragma unroll
+                for (int j = 0; j < NL; ++j) v[j0 + j] = f[j];
+            }
+        };
+        // maxima that the accumulators of the unit's last two chunks, and its sums, are relative to
+        float m0 = -INFINITY, m1 = -INFINITY, ms = -INFINITY;
+        // the unit that ended at chunk q: n chunks, all in D (the last two) and the sums
+        auto finish = [&](int q, const PcbLseTile& t, int nch, int b0) {
+            if (!mbar_wait_bounded(barM + (q & 1), (uint32_t)((q >> 1) & 1))) fail = true;
+            fence_after_sync();
+            fail = fail || slot[1] != 0;
+            const bool in = b0 + s < B, active = b0 + (warp & 3) * 32 < B;
+            const int blocks = ((t.n_rows + 15) & ~15) / EB;
+            const float f1 = nch > 1 ? rescale(m1, m0) : 0.f, fs = nch > 2 ? rescale(ms, m0) : 0.f;
+            const float* ax = MODE != 0 ? aux + (int64_t)t.aux_row * ld + min(b0 + s, B - 1) : nullptr;
+            float* o = out + (int64_t)t.out_row * ld + b0 + s;
+            float a[MODE == 0 ? 1 : EB];
+            auto load_aux = [&](int blk) {
+                if constexpr (MODE != 0) {
+                    if (!active || blk >= blocks) return;
+#pragma unroll
+                    for (int j = 0; j < EB; ++j) a[j] = __ldg(ax + (int64_t)min(blk * EB + j, t.n_rows - 1) * ld);
+                }
+            };
+            load_aux(part);
+#pragma unroll 1
+            for (int blk = part; blk < blocks; blk += 4) {
+                float d[EB];
+                tmem_ld8(d_cols(q) + tlane + blk * EB, d);
+                if (nch > 1) {
+                    float e[EB];
+                    tmem_ld8(d_cols(q - 1) + tlane + blk * EB, e);
+                    wait_ld();
+#pragma unroll
+                    for (int j = 0; j < EB; ++j) d[j] = fmaf(e[j], f1, d[j]);
+                    if (nch > 2) {
+#pragma unroll
+                        for (int j = 0; j < EB; ++j) d[j] = fmaf(sSum[(blk * EB + j) * NS + s], fs, d[j]);
+                    }
+                } else {
+                    wait_ld();
+                }
+                if (MODE == 0) {
+                    float m[EB];
+#pragma unroll
+                    for (int j = 0; j < EB; ++j) m[j] = m0;
+                    log_add<EB, 1>(d, m);
+                } else {
+#pragma unroll
+                    for (int j = 0; j < EB; ++j)
+                        d[j] = m0 == -INFINITY ? 0.f : d[j] * ex2((a[MODE == 0 ? 0 : j] + m0) * kLog2e);
+                    load_aux(blk + 4);
+                }
+                if (fail) {
+#pragma unroll
+                    for (int j = 0; j < EB; ++j) d[j] = __int_as_float(0x7fc00000);
+                }
+                float* dst = o + (int64_t)(blk * EB) * ld;
+                if (in && blk * EB + EB <= t.n_rows) {
+#pragma unroll
+                    for (int j = 0; j < EB; ++j) dst[(int64_t)j * ld] = d[j];
+                } else if (in) {
+#pragma unroll
+                    for (int j = 0; j < EB; ++j)
+                        if (blk * EB + j < t.n_rows) dst[(int64_t)j * ld] = d[j];
+                }
+            }
+        };
+
+        using Z = std::integral_constant<int, 0>;
+        using H = std::integral_constant<int, PT / 2>;
+        PcbLseTile t = {}, tp = {};  // tiles of this unit and of the one before
+        int q = 0, nchp = 0, b0p = 0;
+        if (u0 < u1) {
+            wait_rows(0);
+            load(0, (u0 % num_slices) * NS, tiles[u0 / num_slices].k_cnt, Z{});
+        }
+        for (int u = u0; u < u1; ++u) {
+            t = tiles[u / num_slices];
+            const int nch = chunks_of(t);
+            const int b0 = (u % num_slices) * NS;
+            const bool active = b0 + (warp & 3) * 32 < B;
+            float mrun = -INFINITY;
+            for (int i = 0; i < nch; ++i, ++q) {
+                if (MODE == 2) {
+                    to_log(Z{});
+                    load(q, b0, t.k_cnt, H{});
+                    to_log(H{});
+                }
+                const int nk = t.k_cnt - i * KT - part * PT;  // terms of this part
+                if (!active || nk < PT) {                     // places beyond them count as -inf
+#pragma unroll
+                    for (int j = 0; j < PT; ++j)
+                        if (!active || j >= nk) v[j] = -INFINITY;
+                }
+                float m = v[0];
+#pragma unroll
+                for (int j = 1; j < PT; ++j) m = fmaxf(m, v[j]);
+                float* pm = sPart + (q & 1) * 4 * NS + s;
+                pm[part * NS] = m;
+                asm volatile("bar.sync 1, 512;\n" ::: "memory");
+                m = fmaxf(fmaxf(fmaxf(pm[0], pm[NS]), fmaxf(pm[2 * NS], pm[3 * NS])), mrun);
+                mrun = m;
+                // A's slot: the MMAs of chunk q - 2 have read it
+                if (q >= 2 && !mbar_wait_bounded(barM + (q & 1), (uint32_t)(((q - 2) >> 1) & 1))) fail = true;
+                fence_after_sync();
+                const float mu = m == -INFINITY ? 0.f : m;
+                const uint64_t nmu = pair(-mu, -mu);
+                const uint32_t ta = a_cols(q) + tlane + part * (PT / 2);
+#pragma unroll
+                for (int g = 0; g < PT; g += 16) {
+                    uint32_t hi[8], lo[8];
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) {
+                        const uint64_t x = mul2(add2(pair(v[g + 2 * j], v[g + 2 * j + 1]), nmu), log2e);
+                        const float2 x2 = unpair(x);
+                        const float e0 = ex2(x2.x), e1 = ex2(x2.y);
+                        hi[j] = bf16x2(e0, e1);
+                        if (SPLIT) {
+                            const uint64_t h = pair(__uint_as_float(hi[j] << 16), __uint_as_float(hi[j] & 0xffff0000u));
+                            const float2 l = unpair(fma2(h, minus1, pair(e0, e1)));
+                            lo[j] = bf16x2(l.x, l.y);
+                        }
+                    }
+                    tmem_st8(ta + g / 2, hi);
+                    if (SPLIT) tmem_st8(ta + kColsA + g / 2, lo);
+                }
+                // the next chunk's rows
+                const bool last = i + 1 == nch;
+                if (!last || u + 1 < u1) {
+                    wait_rows(q + 1);
+                    load(q + 1, last ? ((u + 1) % num_slices) * NS : b0, last ? tiles[(u + 1) / num_slices].k_cnt : t.k_cnt, Z{});
+                }
+                // D's slot: what chunk q - 2 left there
+                if (i == 0) {
+                    if (u > u0) finish(q - 1, tp, nchp, b0p);
+                } else if (i >= 2) {
+                    const float f = i > 2 ? rescale(ms, m1) : 0.f;
+                    const int blocks = ((t.n_rows + 15) & ~15) / EB;
+#pragma unroll 1
+                    for (int blk = part; blk < blocks; blk += 4) {
+                        float d[EB];
+                        tmem_ld8(d_cols(q) + tlane + blk * EB, d);
+                        wait_ld();
+#pragma unroll
+                        for (int j = 0; j < EB; ++j) {
+                            float* p = sSum + (blk * EB + j) * NS + s;
+                            *p = i > 2 ? fmaf(*p, f, d[j]) : d[j];
+                        }
+                    }
+                    ms = m1;
+                }
+                m1 = m0;
+                m0 = m;
+                wait_st();
+                fence_before_sync();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(barA + (q & 1));
+            }
+            tp = t;
+            nchp = nch;
+            b0p = b0;
+        }
+        if (u0 < u1) finish(q - 1, tp, nchp, b0p);
+        fence_before_sync();
+    }
+    if (fail) pcb::report_status(status, PCB_STATUS_WAIT_TIMEOUT);
+    __syncthreads();
+    if (warp == kPWarps) {
+        fence_after_sync();
+        tmem_dealloc(taddr, 512);
+    }
+}
+
+template <int MODE, bool SPLIT>
+int launch_persistent(const float* src, const float* src2, const float* aux, float* out, int64_t ld, int B,
+                      const uint8_t* packed, const PcbLseTile* tiles, int num_tiles, int n_max, const int* krow,
+                      const int* chunk_index, int chunk_ld, cudaStream_t s) {
+    const bool sums = chunk_index && chunk_ld > 2;
+    const size_t smem = PSmem(n_max, sums).total;
+    static bool configured[64] = {false};
+    static int sms[64] = {0};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    dev = dev < 0 ? 0 : (dev > 63 ? 63 : dev);
+    if (!configured[dev]) {
+        cudaError_t e = cudaFuncSetAttribute(lse_tmem_persistent_kernel<MODE, SPLIT>,
+                                             cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms[dev], cudaDevAttrMultiProcessorCount, dev);
+        if (e != cudaSuccess) return pcb::set_error(PCB_E_CUDA, "pcb_lse_contract_tmem: %s", cudaGetErrorString(e));
+        configured[dev] = true;
+    }
+    const int slices = (int)pcb::cdiv(B, NS);
+    const int64_t units = (int64_t)num_tiles * slices;
+    if (units > INT32_MAX) return pcb::set_error(PCB_E_ARG, "pcb_lse_contract_tmem: too many tiles");
+    return pcb::launch_status(
+        pcb::launch_k(lse_tmem_persistent_kernel<MODE, SPLIT>, dim3((unsigned)std::min<int64_t>(units, sms[dev])),
+                      dim3(kPThreads), smem, s, 1u, src, src2, aux, out, ld, B, packed, tiles, krow, chunk_index,
+                      chunk_ld, n_max, sums, slices, (int)units, pcb::status_word()),
+        "pcb_lse_contract_tmem");
+}
+
+template <int MODE, bool SPLIT>
+int launch(const float* src, const float* src2, const float* aux, float* out, int64_t ld, int B, const uint8_t* packed,
+           const PcbLseTile* tiles, int num_tiles, int n_max, const int* krow, const int* chunk_index, int chunk_ld,
+           int ksplit, cudaStream_t s) {
+    const bool several = chunk_index && chunk_ld > ksplit;
+    // The CTAs of a cluster wait for one another with their tensor memory allocated, so never
+    // more of them than the tensor memory serves (two) may be resident on an SM.
+    const size_t smem = std::max<size_t>(Smem(n_max, several, ksplit).total, ksplit > 1 ? 77 * 1024 : 0);
+    static bool configured[64] = {false};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    dev = dev < 0 ? 0 : (dev > 63 ? 63 : dev);
+    if (!configured[dev]) {
+        cudaError_t e = cudaFuncSetAttribute(lse_tmem_kernel<MODE, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             227 * 1024);
+        if (e != cudaSuccess) return pcb::set_error(PCB_E_CUDA, "pcb_lse_contract_tmem: %s", cudaGetErrorString(e));
+        configured[dev] = true;
+    }
+    const int slices = (int)pcb::cdiv(B, NS);
+    const int64_t grid = (int64_t)num_tiles * slices * ksplit;
+    if (grid > INT32_MAX) return pcb::set_error(PCB_E_ARG, "pcb_lse_contract_tmem: too many tiles");
+    return pcb::launch_status(
+        pcb::launch_k(lse_tmem_kernel<MODE, SPLIT>, dim3((unsigned)grid), dim3(kThreads), smem, s, (unsigned)ksplit,
+                      src, src2, aux, out, ld, B, packed, tiles, krow, chunk_index, chunk_ld, n_max, several, slices,
+                      pcb::status_word()),
+        "pcb_lse_contract_tmem");
+}
+
+}  // namespace
+
+extern "C" int pcb_lse_contract_tmem(const float* src, const float* src2, const float* aux, float* out, int64_t ld,
+                                     int32_t B, const uint8_t* packed, const PcbLseTile* tiles, int32_t num_tiles,
+                                     int32_t tile_rows, const int32_t* krow, const int32_t* chunk_index,
+                                     int32_t chunk_ld, int32_t mode, int32_t prec, int32_t ksplit, void* stream) {
+    if (!src || !out || !packed || !tiles || !krow || B <= 0 || ld < B || num_tiles < 0 || tile_rows < 1 ||
+        tile_rows > 128 || mode < 0 || mode > 2 || (mode == 2 && !src2) || (mode >= 1 && !aux) || prec < 1 || prec > 2 ||
+        ksplit < 0 || ksplit > kMaxCluster || (chunk_index && chunk_ld < 1) ||
+        (reinterpret_cast<uintptr_t>(packed) & 15) != 0)
+        return pcb::set_error(PCB_E_ARG, "pcb_lse_contract_tmem: bad arguments");
+    if (num_tiles == 0) return PCB_OK;
+    const int n_max = (tile_rows + 15) & ~15;
+    cudaStream_t s = pcb::as_stream(stream);
+    if (ksplit == 0) {
+#define PCB_TP(M) \
+    (prec == 2 ? launch_persistent<M, true>(src, src2, aux, out, ld, B, packed, tiles, num_tiles, n_max, krow, \
+                                            chunk_index, chunk_ld, s) \
+               : launch_persistent<M, false>(src, src2, aux, out, ld, B, packed, tiles, num_tiles, n_max, krow, \
+                                             chunk_index, chunk_ld, s))
+        return mode == 0 ? PCB_TP(0) : (mode == 1 ? PCB_TP(1) : PCB_TP(2));
+#undef PCB_TP
+    }
+#define PCB_TM(M) \
+    (prec == 2 ? launch<M, true>(src, src2, aux, out, ld, B, packed, tiles, num_tiles, n_max, krow, chunk_index, \
+                                 chunk_ld, ksplit, s) \
+               : launch<M, false>(src, src2, aux, out, ld, B, packed, tiles, num_tiles, n_max, krow, chunk_index, \
+                                  chunk_ld, ksplit, s))
+    return mode == 0 ? PCB_TM(0) : (mode == 1 ? PCB_TM(1) : PCB_TM(2));
+#undef PCB_TM
+}

@@ -119,6 +119,40 @@ def _chunk_table(tiles_np: np.ndarray):
     return np.concatenate(parts), ranges
 
 
+def _chunk_index(tiles_np: np.ndarray) -> np.ndarray:
+    """[tiles, chunks]: the position in ``_chunk_table`` of every tile's 128-term chunks (-1: none)."""
+    nch = -(-int(tiles_np[:, 3].max()) // _SHORT_K)
+    index = np.full([tiles_np.shape[0], nch], -1, np.int64)
+    start = 0
+    for j in range(nch):
+        has = np.flatnonzero(tiles_np[:, 3] > _SHORT_K * j)
+        index[has, j] = start + np.arange(has.shape[0])
+        start += has.shape[0]
+    return index
+
+
+def _tmem_ksplit(num_tiles: int, tile_rows: int, num_chunks: int, B: int) -> int:
+    """CTAs (a cluster) that share a tile's chunks in pcb_lse_contract_tmem (``ksplit``). Tiles
+    of more than 64 rows: one per chunk, so that two CTAs fit on an SM (the sums of several
+    chunks take another 64 KB of shared memory); lower tiles: as many as still run at once."""
+    if tile_rows > 64:
+        return num_chunks if num_chunks < 6 else 8
+    return max(1, min(8, num_chunks, 2 * _num_sms() // (num_tiles * -(-B // 128))))
+
+
+class _ShiftedRows:
+    """Rows of a layer's own buffer addressed by circuit row numbers: row ``first`` of the
+    circuit is row 0 of ``rows``. Stands for a tensor in the calls that take row numbers."""
+
+    is_cuda = True
+
+    def __init__(self, rows: torch.Tensor, first: int):
+        self.rows, self.first = rows, first
+
+    def data_ptr(self) -> int:
+        return self.rows.data_ptr() - 4 * self.first * self.rows.stride(0)
+
+
 def _ch_pack(holder: dict, key: str) -> torch.Tensor:
     """The packed-weight buffer of a long-tile chunk table, allocated on the device at first
     use (``holder[key + '_bytes']`` bytes)."""
@@ -203,6 +237,42 @@ def _tc05_chunks(src, src2, aux, out, ld, B, pack, table, ranges, krow, mode, pr
         _tc05_call(src, src2, aux, out, ld, B, pk, t, krow, mode, prec, stream, accum=j > 0)
 
 
+def _tc05_long(src, src2, aux, out, ld, B, pack, table, ranges, krow, mode, prec, stream, holder, plan_key, tiles,
+               tile_rows, index):
+    """A contraction over tiles of any length on the tcgen05 kernels: whole tiles in one launch
+    (pcb_lse_contract_tmem; ``index``: the positions of the chunks of ``tiles`` in ``table`` and
+    ``pack``) or by 128-term chunks (``_tc05_chunks``)."""
+    def tmem(ksplit):
+        nat.call("pcb_lse_contract_tmem", nat.ptr(src), nat.ptr(src2), nat.ptr(aux), nat.ptr(out), ld, B,
+                 nat.ptr(pack), nat.ptr(tiles), tiles.size(0), tile_rows, nat.ptr(krow), nat.ptr(index),
+                 index.size(1), mode, prec, ksplit, stream)
+
+    def chunks():
+        _tc05_chunks(src, src2, aux, out, ld, B, pack, table, ranges, krow, mode, prec, stream, holder, plan_key)
+
+    if prec == 3 or SumLayer.tmem is False:
+        return chunks()
+    if SumLayer.tmem is not None:
+        return tmem(SumLayer.tmem)
+    # One launch of the tensor-memory form, persistent where every SM has a (tile, 128-sample
+    # slice), or by 128-term chunks; the autotuner decides, the first is the static default.
+    # Measured (us, forward, weights packed, graph-timed, chunks / cluster / persistent): 200
+    # regions of 256 x 256, batch 512: 370 / 148 / 88, batch 32: 29.7 / 34.8 / 24.2; one of 2048
+    # x 2048, batch 512: 106 / 77 / 57, batch 64: 17.9 / 28.9 / 53.7; one of 512 x 512, batch 512:
+    # 11.8 / 9.6 / 16.3.
+    ks = _tmem_ksplit(tiles.size(0), tile_rows, index.size(1), B)
+    cands = [("tm", ks), ("tm", 0), ("chunks", 0)]
+    if tiles.size(0) * -(-B // 128) >= _num_sms():
+        cands = [cands[1], cands[0], cands[2]]
+    elif B <= 64:
+        cands = [cands[2], cands[0], cands[1]]
+
+    def run(c):
+        return tmem(c[1]) if c[0] == "tm" else chunks()
+
+    run(TUNER.pick(("long", mode, prec, tiles.size(0), tile_rows, index.size(1), B), cands, run))
+
+
 def _mma(prec: int) -> int:
     """Precision form for the kernels without an E4M3 form (mma.sync, FP32, parameter flows):
     form 3 (E4M3 tcgen05 contractions) runs them in split bf16."""
@@ -214,7 +284,8 @@ def _ws_ok(ld, B, *bufs) -> bool:
     return B % 4 == 0 and ld % 4 == 0 and all(b is None or b.data_ptr() % 16 == 0 for b in bufs)
 
 
-def _tc05_call(src, src2, aux, out, ld, B, pack, tiles, krow, mode, prec, stream, run_rows=0, accum=False):
+def _tc05_call(src, src2, aux, out, ld, B, pack, tiles, krow, mode, prec, stream, run_rows=0, accum=False,
+               tile_rows=128):
     """One tcgen05 contraction: the persistent warp-specialised kernel
     (pcb_lse_contract_tc05_ws, 32- or 64-sample units) or the CTA-per-slice kernel
     (pcb_lse_contract_tc05, 32 or 64 samples and 1 or 2 slices per CTA), chosen by the
@@ -231,7 +302,11 @@ def _tc05_call(src, src2, aux, out, ld, B, pack, tiles, krow, mode, prec, stream
         return
 
     def run(c):
-        if c[0] == "ws":
+        if c[0] == "tm":
+            nat.call("pcb_lse_contract_tmem", nat.ptr(src), nat.ptr(src2), nat.ptr(aux), nat.ptr(out), ld, B,
+                     nat.ptr(pack), nat.ptr(tiles), nt, tile_rows, nat.ptr(krow), nat.ptr(None), 0, mode, prec, c[1],
+                     stream)
+        elif c[0] == "ws":
             nat.call("pcb_lse_contract_tc05_ws", nat.ptr(src), nat.ptr(src2), nat.ptr(aux), nat.ptr(out), ld, B,
                      src.size(0), out.size(0), nat.ptr(pack), nat.ptr(tiles), nt, nat.ptr(krow), mode, prec, c[1],
                      run_rows, 0,
@@ -240,7 +315,10 @@ def _tc05_call(src, src2, aux, out, ld, B, pack, tiles, krow, mode, prec, stream
             nat.call("pcb_lse_contract_tc05", nat.ptr(src), nat.ptr(src2), nat.ptr(aux), nat.ptr(out), ld, B,
                      nat.ptr(pack), nat.ptr(tiles), nt, nat.ptr(krow), mode, prec, c[0], c[1], stream)
 
-    ws_ok = (SumLayer.tc05_ws is not False and prec != 3 and run_rows in (8, 32)
+    shifted = isinstance(src, _ShiftedRows)
+    if prec != 3 and SumLayer.tmem not in (None, False):
+        return run(("tm", min(SumLayer.tmem, 1)))
+    ws_ok = (not shifted and SumLayer.tc05_ws is not False and prec != 3 and run_rows in (8, 32)
              and _ws_ok(ld, B, src, src2, aux, out))
     ws_bt = 32 if mode == 2 or nt * -(-B // 64) < _num_sms() else 64
     if SumLayer.tc05_ws and ws_ok:
@@ -253,6 +331,16 @@ def _tc05_call(src, src2, aux, out, ld, B, pack, tiles, krow, mode, prec, stream
         ws_c = [("ws", ws_bt), ("ws", 96 - ws_bt)]
         # static default: the persistent kernel once the layer has a unit per SM
         cands = ws_c + cands if nt * -(-B // ws_bt) >= _num_sms() else cands + ws_c
+    if prec != 3 and SumLayer.tmem is None:
+        # the tensor-memory form (two CTAs per SM), the default once a 128-sample slice of every
+        # third tile runs per SM; persistent only where every SM has a unit. Measured (us,
+        # forward, graph-timed, best other / two CTAs / persistent): 119 tiles of 128 x 128,
+        # batch 512: 35.8 / 19.2 / 20.5, batch 200: 18.2 / 9.8 / 12.3; 25 tiles, batch 512: 11.3 /
+        # 7.9 / 7.5; 12 tiles: 7.5 / 7.6 / 7.0; 6 tiles: 5.4 / 7.1 / 7.0.
+        units = nt * -(-B // 128)
+        cands = [("tm", 1)] + cands if 3 * units >= _num_sms() else cands + [("tm", 1)]
+        if units >= _num_sms():
+            cands.append(("tm", 0))
     run(TUNER.pick(("tc05", mode, prec, nt, B), cands, run))
 
 
@@ -451,6 +539,13 @@ class SumLayer(Layer):
     tc05_min_tiles = 6    # layers with at least this many tiles use the tcgen05 kernels (BF16 forms)
     tc05_slices_per_cta = None  # sample slices per tcgen05 CTA (None: one)
     tc05_ws = None        # persistent warp-specialised tcgen05 kernel: None autotuned, True forced, False off
+    # contractions with the samples along the tensor-memory lanes (pcb_lse_contract_tmem): None
+    # autotuned against the others, False off, a number that ksplit (0: persistent)
+    tmem = None
+    # node flows x samples from which a backward that may not modify the flows writes log f -
+    # log m to a workspace first (measured, us with / without: 200 regions of 256 x 256, batch 512:
+    # 468 / 610; 119 of 128 x 128: 104 / 109; 25 of 128 x 128: 97 / 82, bound by the host)
+    ratio_min_values = 1 << 22
     tc05_long = True      # tiles of more than 128 terms as accumulating tcgen05 chunks (BF16 / E4M3 forms)
     chunk_partials = True  # all chunks of a layer in one launch into partial rows, then pcb_chunk_combine
     # The single-stage kernels of small layers read pre-packed weights too (the circuit packs
@@ -583,6 +678,7 @@ class SumLayer(Layer):
             ech_t = _chunk_table(tiles_np)
             el_groups.append(dict(
                 ch=None if ech_t is None else _i32(ech_t[0]), ch_ranges=None if ech_t is None else ech_t[1],
+                ch_index=None if ech_t is None else _i32(_chunk_index(tiles_np)),
                 ch_pack=None, ch_pack_bytes=0 if ech_t is None else ech_t[0].shape[0] * _PACK_BYTES,
                 cbs=cbs, tm=_tile_rows(max(t[1] for t in tiles)), tiles=_i32(tiles_np),
                 krow=_i32(np.concatenate(klist)), kw=_i32(kw_np),
@@ -595,6 +691,7 @@ class SumLayer(Layer):
         fch = _chunk_table(fw_np)
         return dict(
             fw_ch=None if fch is None else _i32(fch[0]), fw_ch_ranges=None if fch is None else fch[1],
+            fw_ch_index=None if fch is None else _i32(_chunk_index(fw_np)),
             fw_ch_pack=None, fw_ch_pack_bytes=0 if fch is None else fch[0].shape[0] * _PACK_BYTES,
             fw_tiles=_i32(fw_np), fw_tm=fw_tm, fw_run=_run_rows(fw_np, krow_c),
             fw_short=bool(fw_np.shape[0]) and int(fw_np[:, 3].max()) <= _SHORT_K,
@@ -783,13 +880,14 @@ class SumLayer(Layer):
                 self.pack_forward_weights(params, B, force_use_bf16, force_use_fp32)
                 _weights_packed = True
             _tc05_call(element_mars, None, None, node_mars, ld, B, d["fw_pack"], t, d["krow"], 0, prec, st,
-                       d["fw_run"])
+                       d["fw_run"], tile_rows=d["fw_tm"])
             return
         if self._fw_long(d, prec):
             if not _weights_packed:
                 self.pack_forward_weights(params, B, force_use_bf16, force_use_fp32)
-            _tc05_chunks(element_mars, None, None, node_mars, ld, B, _ch_pack(d, "fw_ch_pack"), d["fw_ch"], d["fw_ch_ranges"],
-                         d["krow"], 0, prec, st, holder=d, plan_key="fw_ch_plan")
+            _tc05_long(element_mars, None, None, node_mars, ld, B, _ch_pack(d, "fw_ch_pack"), d["fw_ch"],
+                       d["fw_ch_ranges"], d["krow"], 0, prec, st, holder=d, plan_key="fw_ch_plan", tiles=t,
+                       tile_rows=d["fw_tm"], index=d["fw_ch_index"])
             return
         prec = _mma(prec)
         # _fuse_fw = (term_children, element values out): the product layer below is fused in
@@ -847,6 +945,19 @@ class SumLayer(Layer):
         if allow_modify_flows and not kwargs.get("_flows_modified"):
             nat.call("pcb_modify_flows", nat.ptr(node_flows), nat.ptr(node_mars), ld, B, self._layer_nid_range[0],
                      self._layer_nid_range[1], nat.stream())
+        flows, modified = node_flows, allow_modify_flows
+        if (not allow_modify_flows and kwargs.get("_pflow_stream") is None and kwargs.get("_fuse_bw") is None
+                and not force_use_fp32 and SumLayer.bf16_form != 3
+                and (self._layer_nid_range[1] - self._layer_nid_range[0]) * B >= SumLayer.ratio_min_values
+                and all(self._el_tc05(eg, p) or self._el_long(eg, p)
+                                                    for eg in d["el_groups"] for p in (self._el_prec(eg, B, False),))):
+            # log f - log m of this layer's nodes once, in a workspace, instead of in every tile
+            # of both contractions that reads them (node_flows stays as the caller has it)
+            lo, hi = self._layer_nid_range
+            ratios = torch.empty([hi - lo, ld], dtype=torch.float32, device=node_flows.device)
+            nat.call("pcb_flow_ratios", nat.ptr(node_flows), nat.ptr(node_mars), nat.ptr(ratios), ld, B, lo, hi,
+                     nat.stream())
+            flows, modified = _ShiftedRows(ratios, lo), True
         skip = kwargs.get("_pflow_skip")
         if skip and id(self) in skip:  # the circuit launches them once for this layer's tied set
             param_flows = None
@@ -868,13 +979,14 @@ class SumLayer(Layer):
             prec = self._el_prec(eg, B, force_use_fp32)
             if self._el_tc05(eg, prec):
                 st = nat.stream()
-                _tc05_call(node_flows, None if allow_modify_flows else node_mars, element_mars, element_flows, ld, B,
-                           eg["pack"], et, eg["krow"], 1 if allow_modify_flows else 2, prec, st, eg["run"])
+                _tc05_call(flows, None if modified else node_mars, element_mars, element_flows, ld, B,
+                           eg["pack"], et, eg["krow"], 1 if modified else 2, prec, st, eg["run"], tile_rows=eg["tm"])
                 continue
             if self._el_long(eg, prec):
-                _tc05_chunks(node_flows, None if allow_modify_flows else node_mars, element_mars, element_flows, ld,
-                             B, _ch_pack(eg, "ch_pack"), eg["ch"], eg["ch_ranges"], eg["krow"], 1 if allow_modify_flows else 2,
-                             prec, nat.stream(), holder=eg, plan_key="ch_plan")
+                _tc05_long(flows, None if modified else node_mars, element_mars, element_flows, ld, B,
+                           _ch_pack(eg, "ch_pack"), eg["ch"], eg["ch_ranges"], eg["krow"], 1 if modified else 2,
+                           prec, nat.stream(), holder=eg, plan_key="ch_plan", tiles=et, tile_rows=eg["tm"],
+                           index=eg["ch_index"])
                 continue
             prec = _mma(prec)
             if eg["short"] and SumLayer.short_kernels:
@@ -908,8 +1020,7 @@ class SumLayer(Layer):
             if ready is not None:
                 pflow_stream.wait_event(ready)
             with torch.cuda.stream(pflow_stream if ready is not None else torch.cuda.current_stream()):
-                self.param_flows_only(node_flows, node_mars, element_mars, params, param_flows,
-                                      allow_modify_flows=allow_modify_flows, force_use_fp32=force_use_fp32)
+                self._param_flows(flows, node_mars, element_mars, params, param_flows, modified, force_use_fp32)
 
     def _backward_partial(self, part, node_flows, element_flows, node_mars, element_mars, params, param_flows,
                           force_use_fp32):
@@ -967,12 +1078,18 @@ class SumLayer(Layer):
                          force_use_fp32: bool = False) -> None:
         """Accumulate this layer's parameter flows on the current stream (``allow_modify_flows``:
         node_flows already hold log f - log m for this layer's nodes)."""
-        d = self._desc(node_mars.device)
         B = node_mars.size(1)
         ld = node_mars.stride(0)
         for t in (node_flows, element_mars):
             if t.size(1) != B or t.stride(0) != ld or t.stride(1) != 1:
                 raise ValueError("node flows, node values and element values must share one [rows, B] layout")
+        self._param_flows(node_flows, node_mars, element_mars, params, param_flows, allow_modify_flows, force_use_fp32)
+
+    def _param_flows(self, node_flows, node_mars, element_mars, params, param_flows, allow_modify_flows, force_use_fp32):
+        """``param_flows_only`` after its checks; ``node_flows`` may be a ``_ShiftedRows``."""
+        d = self._desc(node_mars.device)
+        B = node_mars.size(1)
+        ld = node_mars.stride(0)
         prec = 0 if force_use_fp32 or B < 16 else _mma(SumLayer.bf16_form)
         st = nat.stream()
 

@@ -1,0 +1,86 @@
+"""Contractions with the samples along the tensor-memory lanes (pcb_lse_contract_tmem) against
+FP64: every launch form, at the edges of its tiles, chunks, slices and clusters."""
+
+import pytest
+import torch
+
+import pyjuice_b200 as juice
+from pyjuice_b200 import _native as nat
+from pyjuice_b200.layer.layers import SumLayer
+from pyjuice_b200.nodes.distributions import Categorical
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture
+def settings():
+    names = ("tmem", "tc05_min_tiles", "bf16_form", "ratio_min_values")
+    saved = {n: getattr(SumLayer, n) for n in names}
+    yield
+    for n, v in saved.items():
+        setattr(SumLayer, n, v)
+
+
+def _layer(regions, nodes, terms, bs, device):
+    with juice.set_block_size(bs):
+        leaves = [juice.inputs(v, num_node_blocks=terms // bs, dist=Categorical(num_cats=2)) for v in range(2 * regions)]
+        prods = [juice.multiply(leaves[2 * r], leaves[2 * r + 1]) for r in range(regions)]
+        sums = [juice.summate(p, num_node_blocks=nodes // bs) for p in prods]
+    juice.InputLayer(leaves, cum_nodes=bs)
+    juice.ProdLayer(prods)
+    return juice.SumLayer(sums, global_nid_start=bs, global_pid_start=bs ** 2, global_pfid_start=0,
+                          node2tiednodes=dict()).to(device)
+
+
+# regions, nodes, terms, block, batch, ksplit (0: persistent), bf16 form
+CASES = [(1, 16, 16, 16, 16, 1, 2), (3, 16, 128, 16, 129, 0, 2), (2, 144, 96, 16, 127, 1, 2), (2, 128, 128, 32, 128, 0, 1),
+         (1, 64, 144, 16, 257, 1, 2), (2, 128, 256, 32, 130, 2, 2), (1, 96, 400, 16, 33, 3, 2), (1, 128, 640, 32, 200, 5, 2),
+         (1, 48, 1040, 16, 100, 8, 2), (5, 128, 256, 32, 300, 0, 2), (3, 80, 656, 16, 140, 0, 2), (160, 32, 32, 32, 512, 0, 2),
+         (40, 256, 256, 32, 260, 0, 2), (2, 128, 272, 16, 64, 8, 1)]
+
+
+@pytest.mark.parametrize("regions,nodes,terms,bs,B,ksplit,form", CASES)
+def test_contractions(regions, nodes, terms, bs, B, ksplit, form, cuda_device, settings):
+    """Values and element flows (modified, unmodified through the kernel and through the ratio
+    workspace), with samples that have no term above -inf and flows of zero."""
+    SumLayer.tmem, SumLayer.tc05_min_tiles, SumLayer.bf16_form = ksplit, 1, form
+    layer = _layer(regions, nodes, terms, bs, cuda_device)
+    gen = torch.Generator(device=cuda_device).manual_seed(nodes + terms + B)
+    rnd = lambda *shape: torch.rand(shape, generator=gen, device=cuda_device)
+    w = torch.exp(-4.0 * rnd(regions, nodes, terms))
+    w = w / w.sum(dim=2, keepdim=True)
+    params = torch.cat([torch.zeros([bs ** 2], device=cuda_device),
+                        w.reshape(regions, nodes // bs, bs, terms).permute(0, 1, 3, 2).reshape(-1)])
+    em = -12.0 * rnd(regions, terms, B)
+    em[rnd(regions, terms, B) < 0.1] = -float("inf")
+    em[0, :, 0] = -float("inf")  # a sample without any
+    ems = torch.cat([torch.full([bs, B], -float("inf"), device=cuda_device), em.reshape(-1, B)])
+    nm = torch.full([bs + regions * nodes, B], 5.0, device=cuda_device)
+    layer(nm, ems, params, force_use_bf16=True)
+    ref = torch.log(w.double() @ em.double().exp())
+    got = nm[bs:].reshape(regions, nodes, B).double()
+    # operand rounding: split products are within 3 * 2^-18, single ones within 2^-8 + 2^-16;
+    # 24 accumulations of 2^-23 and the approximations' 2^-21 stay below the rest of the bound
+    tol = 2e-5 if form == 2 else 5e-3
+    assert torch.equal(torch.isinf(got), torch.isinf(ref))
+    fin = torch.isfinite(ref)
+    assert torch.all((got - ref)[fin].abs() <= tol + 4e-7 * ref[fin].abs())
+    assert torch.all(nm[:bs] == 5.0)
+    nm64 = ref.float().double()
+    nms = torch.cat([torch.zeros([bs, B], device=cuda_device), ref.float().reshape(-1, B)])
+    nf = torch.softmax(3.0 * rnd(regions, nodes, B), dim=1)
+    nf[rnd(regions, nodes, B) < 0.1] = 0.0
+    nfs = torch.cat([torch.zeros([bs, B], device=cuda_device), nf.reshape(-1, B)])
+    ratio = torch.where(torch.isfinite(nm64), nf.double() * torch.exp(-nm64), 0.0)
+    want = (w.double().transpose(1, 2) @ ratio) * em.double().exp()
+    for modify, ratios in ((False, 1 << 62), (False, 0), (True, 0)):
+        SumLayer.ratio_min_values = ratios
+        flows = nfs.clone()
+        ef = torch.full_like(ems, 9.0)
+        layer.backward(flows, ef, nms, ems, params, None, allow_modify_flows=modify)
+        assert modify or torch.equal(flows, nfs)
+        out = ef[bs:].reshape(regions, terms, B).double()
+        # as above, and exponents of magnitude up to about 30 rounded three times
+        assert torch.all((out - want).abs() <= (tol + 1e-5) * want)
+        assert torch.all(ef[:bs] == 9.0)
+    assert nat.device_status() == 0
