@@ -550,6 +550,17 @@ int pcb_sum_pflows(const float* node_flows, const float* node_mars, const float*
                    int32_t modified, int32_t atomic, int32_t tile_children, int32_t prec, void* stream);
 
 /*
+ * pcb_sum_pflows_tc05 (prec 1, 2) with one sample per lane: each tile (tile_children 64 or
+ * 128) contracts the whole batch in one CTA, for layers of many tiles or small batches. Rows
+ * need no alignment. Replaces the same reference kernels (sum_layer.py:2052-2282).
+ */
+int pcb_sum_pflows_lanes(const float* node_flows, const float* node_mars, const float* element_mars, int64_t ld,
+                         int32_t B, const float* params, float* param_flows, const PcbPflowTile* tiles,
+                         int32_t num_tiles, int32_t rows_per_block, const int32_t* cids, const int32_t* pids,
+                         const int32_t* pfids, int32_t modified, int32_t atomic, int32_t tile_children, int32_t prec,
+                         void* stream);
+
+/*
  * pcb_sum_pflows on the tcgen05 tensor cores (prec 1: bf16 operands, 2: split bf16 hi + lo,
  * three MMAs; tile_children 64 or 128): the [128 x tile_children] accumulator of a tile stays
  * in tensor memory over the CTA's batch slice; each 32-sample chunk is exponentiated into

@@ -1096,7 +1096,7 @@ class SumLayer(Layer):
         def run(c, target):
             tc05, kc = c
             pt = d[{128: "pf_tiles128", 64: "pf_tiles", 32: "pf_tiles32"}[kc]]
-            nat.call("pcb_sum_pflows_tc05" if tc05 else "pcb_sum_pflows", nat.ptr(node_flows), nat.ptr(node_mars),
+            nat.call("pcb_sum_pflows_lanes" if tc05 == "lanes" else "pcb_sum_pflows_tc05" if tc05 else "pcb_sum_pflows", nat.ptr(node_flows), nat.ptr(node_mars),
                      nat.ptr(element_mars), ld, B, nat.ptr(params), nat.ptr(target), nat.ptr(pt), pt.size(0),
                      self.block_size, nat.ptr(d["krow"]), nat.ptr(d["kw"]), nat.ptr(d["kpf"]),
                      1 if allow_modify_flows else 0, 1 if self._has_tied else 0, kc, prec, st)
@@ -1108,6 +1108,16 @@ class SumLayer(Layer):
             kcs = (kc_fixed,) if kc_fixed else (64, 128, 32)
             tcs = (tc_fixed,) if tc_fixed is not None else (True, False)
             cands = [(t, k) for t in tcs for k in kcs if not (t and k == 32)]
+            n64, n128 = d["pf_tiles"].size(0), d["pf_tiles128"].size(0)
+            if tc_fixed is None and kc_fixed is None and (B <= 64 or n64 > _num_sms()):
+                # One sample per lane, also the static default: for short batches, and where the
+                # others would not split the batch over a cluster (sums over a part of the batch
+                # are truncated less). Measured (us, rewritten flows, best other / 64 / 128
+                # children per tile): 200 regions of 256 x 256, batch 512: 245 / 163 / 117, batch
+                # 64: 89 / 54 / 45; 119 of 128 x 128, batch 512: 46.5 / 29.6 / 36.0; one of 2048 x
+                # 2048, batch 512: 83.5 / 52.8 / 36.9; 25 of 128 x 128, batch 64: 11.8 / 6.5 / 8.9.
+                lanes = [("lanes", 128), ("lanes", 64)] if n128 < n64 else [("lanes", 64)]
+                cands = (lanes if n128 >= _num_sms() else lanes[::-1]) + cands
         if len(cands) == 1:
             return run(cands[0], param_flows)
         # candidates accumulate into a scratch copy while they are timed

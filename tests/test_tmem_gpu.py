@@ -84,3 +84,40 @@ def test_contractions(regions, nodes, terms, bs, B, ksplit, form, cuda_device, s
         assert torch.all((out - want).abs() <= (tol + 1e-5) * want)
         assert torch.all(ef[:bs] == 9.0)
     assert nat.device_status() == 0
+
+
+@pytest.mark.parametrize("nodes,terms,bs,B,form", [(16, 16, 16, 1, 2), (128, 64, 32, 64, 2), (144, 80, 16, 65, 2), (256, 256, 32, 257, 2),
+                                                   (48, 200, 8, 511, 2), (64, 128, 64, 130, 1)])
+@pytest.mark.parametrize("children", [64, 128])
+@pytest.mark.parametrize("modified", [False, True])
+def test_lane_parameter_flows(nodes, terms, bs, B, form, children, modified, cuda_device):
+    """pcb_sum_pflows_lanes: flows added to the slots, for tiles with fewer rows or children than
+    a full one, the last samples of a chunk, zero flows and children without value."""
+    layer = _layer(2, nodes, terms, bs, cuda_device)
+    d = layer._desc(torch.device(cuda_device))
+    gen = torch.Generator(device=cuda_device).manual_seed(nodes + B)
+    rnd = lambda *shape: torch.rand(shape, generator=gen, device=cuda_device)
+    w = rnd(2, nodes, terms) + 0.01
+    pack = lambda x: x.reshape(2, nodes // bs, bs, terms).permute(0, 1, 3, 2).reshape(-1)
+    params = torch.cat([torch.zeros([bs ** 2], device=cuda_device), pack(w)])
+    em = -8.0 * rnd(2, terms, B)
+    em[rnd(2, terms, B) < 0.1] = -float("inf")
+    nm = -8.0 * rnd(2, nodes, B)
+    nf = rnd(2, nodes, B)
+    nf[rnd(2, nodes, B) < 0.1] = 0.0
+    pad = lambda x, v: torch.cat([torch.full([bs, B], v, device=cuda_device), x.reshape(-1, B)])
+    ems, nms = pad(em, -float("inf")), pad(nm, 0.0)
+    flows = pad(nf.log() - nm, 0.0) if modified else pad(nf, 0.0)
+    old = rnd(2 * nodes * terms)
+    pf = old.clone()
+    tiles = d["pf_tiles" if children == 64 else "pf_tiles128"]
+    nat.call("pcb_sum_pflows_lanes", nat.ptr(flows), nat.ptr(nms), nat.ptr(ems), B, B, nat.ptr(params), nat.ptr(pf),
+             nat.ptr(tiles), tiles.size(0), bs, nat.ptr(d["krow"]), nat.ptr(d["kw"]), nat.ptr(d["kpf"]),
+             1 if modified else 0, 0, children, form, nat.stream())
+    ratio = nf.double() * torch.exp(-nm.double())
+    want = pack(w.double() * (ratio @ em.double().exp().transpose(1, 2)))
+    # split operands: products within 3 * 2^-18; 36 accumulations truncated by 2^-23; exponents of
+    # magnitude up to 24 rounded three times; the sum with the old value rounded once
+    tol = (3.0 * 2.0 ** -18 if form == 2 else 2.0 ** -7) + 36 * 2.0 ** -23 + 1e-5
+    assert torch.all((pf.double() - old.double() - want).abs() <= tol * want + 2.0 ** -23 * (old.double() + want))
+    assert nat.device_status() == 0
