@@ -40,7 +40,7 @@ class Autotuner:
 
     @staticmethod
     def _key(key: Sequence[Hashable]) -> str:
-        return "|".join(str(k) for k in key)
+        return "|".join(map(str, key))
 
     def pick(self, key: Sequence[Hashable], candidates: Sequence, run: Callable[[object], None]):
         """The chosen candidate for ``key`` (timing ``run(candidate)`` for each candidate on the

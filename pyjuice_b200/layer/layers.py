@@ -1019,7 +1019,9 @@ class SumLayer(Layer):
         if param_flows is not None:
             if ready is not None:
                 pflow_stream.wait_event(ready)
-            with torch.cuda.stream(pflow_stream if ready is not None else torch.cuda.current_stream()):
+                with torch.cuda.stream(pflow_stream):
+                    self._param_flows(flows, node_mars, element_mars, params, param_flows, modified, force_use_fp32)
+            else:
                 self._param_flows(flows, node_mars, element_mars, params, param_flows, modified, force_use_fp32)
 
     def _backward_partial(self, part, node_flows, element_flows, node_mars, element_mars, params, param_flows,
