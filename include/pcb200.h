@@ -365,6 +365,13 @@ int pcb_pack_weights(const float* params, const PcbLseTile* tiles, int32_t num_t
                      const int32_t* kw, int32_t w_stride, uint8_t* packed, void* stream);
 
 /*
+ * The weights of the same tiles in three bf16 parts (hi, mid, lo: 24 bits), 98304 bytes per
+ * tile: the operand of pcb_lse_contract_tmem's FP32 form.
+ */
+int pcb_pack_weights_f32(const float* params, const PcbLseTile* tiles, int32_t num_tiles, int32_t rows_per_block,
+                         const int32_t* kw, int32_t w_stride, uint8_t* packed, void* stream);
+
+/*
  * The same weights packed for the E4M3 form of pcb_lse_contract_tc05 (prec 3): for tile t,
  * at packed + t * 65536, 16384 bytes of e4m3 values W(k, r) * 448 / max_k W(k, r) in the
  * K-major no-swizzle layout of a 128 x 128 8-bit operand (core matrices of 8 rows x 16
@@ -388,14 +395,14 @@ typedef struct {
     int32_t num_tiles;
     int32_t rows_per_block_log2;
     int32_t w_stride;
-    int32_t format;              /* 0: bf16 hi + lo (pcb_pack_weights), 1: e4m3 (pcb_pack_weights_fp8) */
+    int32_t format;              /* 0: bf16 hi + lo (pcb_pack_weights), 1: e4m3 (.._fp8), 2: three parts (.._f32) */
 } PcbPackJob;
 
 /*
  * pcb_pack_weights for several tile tables in one launch (device arrays): global tile g
  * (g < total_tiles) is tile tile_index[g] of jobs[tile_job[g]]. The caller guarantees
  * tile_index[g] < that job's num_tiles. Same output as one pcb_pack_weights (format 0) or
- * pcb_pack_weights_fp8 (format 1) per job.
+ * pcb_pack_weights_fp8 (format 1) or pcb_pack_weights_f32 (format 2) per job.
  * No counterpart in the reference (see pcb_pack_weights).
  */
 int pcb_pack_weights_multi(const float* params, const PcbPackJob* jobs, const int32_t* tile_job,
@@ -434,12 +441,15 @@ int pcb_lse_contract_tc05_accum(const float* src, const float* src2, const float
                                 int32_t slices_per_cta, void* stream);
 
 /*
- * pcb_lse_contract in its BF16 forms (prec 1: single operands, 2: split) for tiles of any
- * number of terms, in one launch, with the samples along the tensor-memory lanes. `packed`
+ * pcb_lse_contract for tiles of any number of terms, in one launch, with the samples along the
+ * tensor-memory lanes: the BF16 forms (prec 1: single operands, 2: split), and, persistent
+ * (ksplit 0) for modes 0 and 1, the plain FP32 form (prec 0, operands in three parts packed by
+ * pcb_pack_weights_f32, 98304 bytes per tile). `packed`
  * holds the tiles' weights (pcb_pack_weights): of tile t itself (chunk_index NULL, tiles of
  * at most 128 terms), or of its 128-term chunk j at packed + chunk_index[t * chunk_ld + j] *
  * 65536 (chunk_ld: at least the chunks of every tile). `tile_rows`: at least the rows of
- * every tile (<= 128). ksplit (1 .. 8): CTAs (a cluster) that share a tile's chunks. Rows of src, src2, aux and out need no alignment.
+ * every tile (<= 128). ksplit 0: persistent, one CTA per SM
+ * over all (tile, 128-sample slice) units; 1 .. 8: CTAs (a cluster) that share a tile's chunks. Rows of src, src2, aux and out need no alignment.
  * Replaces the same reference kernels as pcb_lse_contract (sum_layer.py:454-568,
  * 1572-1730).
  */

@@ -183,7 +183,7 @@ constexpr int kPackSplit = (128 * (KT / 8)) / 256;
 
 __device__ __forceinline__ void pack_tile_part(const float* __restrict__ params, const PcbLseTile& t, int rpb_log2,
                                                const int* __restrict__ kw, int w_stride, uint8_t* __restrict__ dst,
-                                               int part) {
+                                               int part, bool three = false) {
     // Rows up to the next multiple of 32 (the accumulators of others are never used), all terms
     // (zeros behind the tile's, which meet zero exponentials in the contractions).
     const int rpb_mask = (1 << rpb_log2) - 1;
@@ -215,6 +215,13 @@ __device__ __forceinline__ void pack_tile_part(const float* __restrict__ params,
     split8(w, h, l);
     const uint32_t off = (uint32_t)(r >> 3) * kSBO + (uint32_t)kg * kLBO + (uint32_t)(r & 7) * 16;
     *reinterpret_cast<uint4*>(dst + off) = h;
+    if (three) {  // FP32 form: what hi leaves, split once more
+#pragma unroll
+        for (int j = 0; j < 8; ++j) w[j] -= __bfloat162float(__float2bfloat16_rn(w[j]));
+        uint4 lo;
+        split8(w, l, lo);
+        *reinterpret_cast<uint4*>(dst + 2 * kHalfBytes + off) = lo;
+    }
     *reinterpret_cast<uint4*>(dst + kHalfBytes + off) = l;
 }
 
@@ -266,11 +273,11 @@ pack_weights_fp8_kernel(const float* __restrict__ params, const PcbLseTile* __re
 
 __global__ void __launch_bounds__(256)
 pack_weights_kernel(const float* __restrict__ params, const PcbLseTile* __restrict__ tiles, int rpb_log2,
-                    const int* __restrict__ kw, int w_stride, uint8_t* __restrict__ packed) {
+                    const int* __restrict__ kw, int w_stride, uint8_t* __restrict__ packed, bool three) {
     pcb::pdl_begin();
     const int tile = blockIdx.x / kPackSplit;
-    pack_tile_part(params, tiles[tile], rpb_log2, kw, w_stride, packed + (size_t)tile * kTileBytes,
-                   blockIdx.x % kPackSplit);
+    pack_tile_part(params, tiles[tile], rpb_log2, kw, w_stride,
+                   packed + (size_t)tile * (three ? 3 * kHalfBytes : kTileBytes), blockIdx.x % kPackSplit, three);
 }
 
 // All tiles of several tile tables in one launch: global tile g is tile tile_index[g] of
@@ -289,8 +296,9 @@ pack_weights_multi_kernel(const float* __restrict__ params, const PcbPackJob* __
                           jb.packed + (size_t)ti * kTileBytes, smax);
         return;
     }
+    const bool three = jb.format == 2;
     pack_tile_part(params, jb.tiles[ti], jb.rows_per_block_log2, jb.kw, jb.w_stride,
-                   jb.packed + (size_t)ti * kTileBytes, blockIdx.x % kPackSplit);
+                   jb.packed + (size_t)ti * (three ? 3 * kHalfBytes : kTileBytes), blockIdx.x % kPackSplit, three);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -1223,19 +1231,32 @@ int launch_n(int mode, int prec, int num_tiles, int spc, const float* src, const
 
 }  // namespace
 
+static int pack_entry(const char* name, const float* params, const PcbLseTile* tiles, int32_t num_tiles,
+                      int32_t rows_per_block, const int32_t* kw, int32_t w_stride, uint8_t* packed, void* stream,
+                      bool three) {
+    if (!params || !tiles || !kw || !packed || num_tiles < 0 || rows_per_block <= 0 ||
+        (rows_per_block & (rows_per_block - 1)) || (reinterpret_cast<uintptr_t>(packed) & 15) != 0)
+        return pcb::set_error(PCB_E_ARG, "%s: bad arguments", name);
+    if (num_tiles == 0) return PCB_OK;
+    if ((int64_t)num_tiles * kPackSplit > 2147483647) return pcb::set_error(PCB_E_ARG, "%s: too many tiles", name);
+    int rpb_log2 = 0;
+    while ((1 << rpb_log2) < rows_per_block) ++rpb_log2;
+    return pcb::launch_status(pcb::launch_k(pack_weights_kernel, dim3((unsigned)(num_tiles * kPackSplit)), dim3(256), 0,
+                                            pcb::as_stream(stream), 1u, params, tiles, rpb_log2, kw, w_stride, packed,
+                                            three), name);
+}
+
 extern "C" int pcb_pack_weights(const float* params, const PcbLseTile* tiles, int32_t num_tiles,
                                 int32_t rows_per_block, const int32_t* kw, int32_t w_stride, uint8_t* packed,
                                 void* stream) {
-    if (!params || !tiles || !kw || !packed || num_tiles < 0 || rows_per_block <= 0 ||
-        (rows_per_block & (rows_per_block - 1)) || (reinterpret_cast<uintptr_t>(packed) & 15) != 0)
-        return pcb::set_error(PCB_E_ARG, "pcb_pack_weights: bad arguments");
-    if (num_tiles == 0) return PCB_OK;
-    int rpb_log2 = 0;
-    while ((1 << rpb_log2) < rows_per_block) ++rpb_log2;
-    if ((int64_t)num_tiles * kPackSplit > 2147483647) return pcb::set_error(PCB_E_ARG, "pcb_pack_weights: too many tiles");
-    return pcb::launch_status(pcb::launch_k(pack_weights_kernel, dim3((unsigned)(num_tiles * kPackSplit)), dim3(256),
-                                            0, pcb::as_stream(stream), 1u, params, tiles, rpb_log2, kw, w_stride,
-                                            packed), "pcb_pack_weights");
+    return pack_entry("pcb_pack_weights", params, tiles, num_tiles, rows_per_block, kw, w_stride, packed, stream, false);
+}
+
+extern "C" int pcb_pack_weights_f32(const float* params, const PcbLseTile* tiles, int32_t num_tiles,
+                                    int32_t rows_per_block, const int32_t* kw, int32_t w_stride, uint8_t* packed,
+                                    void* stream) {
+    return pack_entry("pcb_pack_weights_f32", params, tiles, num_tiles, rows_per_block, kw, w_stride, packed, stream,
+                      true);
 }
 
 extern "C" int pcb_pack_weights_fp8(const float* params, const PcbLseTile* tiles, int32_t num_tiles,

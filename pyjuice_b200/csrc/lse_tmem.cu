@@ -201,30 +201,48 @@ __device__ __forceinline__ uint32_t idesc_n(int n) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
 }
 
-// The MMAs of one chunk into a fresh accumulator d (a: A's hi columns, lo behind them; w, wl: the
-// weights' hi and lo). Tiles of several chunks take the small products first: what additions
-// to an already large accumulator truncate is then left by the hi * hi steps alone. Tiles of one
-// chunk take them step by step, like the other tcgen05 kernels, whose results theirs equal.
-template <bool SPLIT>
-__device__ __forceinline__ void issue_mmas(uint32_t d, uint32_t a, uint32_t w, uint32_t wl, int steps, uint32_t idesc,
+// The MMAs of one chunk into a fresh accumulator d (a: A's parts, kColsA columns apart; w: the
+// weights' parts, wp bytes apart). Tiles of several chunks, and the FP32 form, take the small
+// products first: what additions to an already large accumulator truncate is then left by the
+// hi * hi steps alone. Split tiles of one chunk take them step by step, like the other tcgen05
+// kernels, whose results theirs equal. The FP32 form halves what truncation is left with a
+// second accumulator.
+template <int NP>
+__device__ __forceinline__ void issue_mmas(uint32_t d, uint32_t a, uint32_t w, uint32_t wp, int steps, uint32_t idesc,
                                            bool small_first) {
-    if (!SPLIT || !small_first) {
+    auto mma = [&](int s, int pa, int pw, uint32_t acc, uint32_t dd) {
+        mma_ts(dd, a + pa * kColsA + s * 8, desc(w + pw * wp + (uint32_t)s * 2 * kLBO, kLBO, kSBO), idesc, acc);
+    };
+    if (NP == 3) {
+        // half of the hi * hi steps to the accumulator behind d, alone
+        const uint32_t d2 = d + kColsD;
+        const int h = (steps + 1) / 2;
         for (int s = 0; s < steps; ++s) {
-            const uint32_t o = (uint32_t)s * 2 * kLBO;
-            mma_ts(d, a + s * 8, desc(w + o, kLBO, kSBO), idesc, s > 0 ? 1u : 0u);
-            if (SPLIT) {
-                mma_ts(d, a + s * 8, desc(wl + o, kLBO, kSBO), idesc, 1u);
-                mma_ts(d, a + kColsA + s * 8, desc(w + o, kLBO, kSBO), idesc, 1u);
+            mma(s, 0, 2, s > 0 ? 1u : 0u, d);
+            mma(s, 2, 0, 1u, d);
+            mma(s, 1, 1, 1u, d);
+        }
+        for (int s = 0; s < steps; ++s) {
+            mma(s, 0, 1, 1u, d);
+            mma(s, 1, 0, 1u, d);
+        }
+        for (int s = 0; s < h; ++s) mma(s, 0, 0, s > 0 ? 1u : 0u, d2);
+        for (int s = h; s < steps; ++s) mma(s, 0, 0, 1u, d);
+    } else if (NP == 1 || !small_first) {
+        for (int s = 0; s < steps; ++s) {
+            mma(s, 0, 0, s > 0 ? 1u : 0u, d);
+            if (NP == 2) {
+                mma(s, 0, 1, 1u, d);
+                mma(s, 1, 0, 1u, d);
             }
         }
-        return;
+    } else {
+        for (int s = 0; s < steps; ++s) {
+            mma(s, 0, 1, s > 0 ? 1u : 0u, d);
+            mma(s, 1, 0, 1u, d);
+        }
+        for (int s = 0; s < steps; ++s) mma(s, 0, 0, 1u, d);
     }
-    for (int s = 0; s < steps; ++s) {
-        const uint32_t o = (uint32_t)s * 2 * kLBO;
-        mma_ts(d, a + s * 8, desc(wl + o, kLBO, kSBO), idesc, s > 0 ? 1u : 0u);
-        mma_ts(d, a + kColsA + s * 8, desc(w + o, kLBO, kSBO), idesc, 1u);
-    }
-    for (int s = 0; s < steps; ++s) mma_ts(d, a + s * 8, desc(w + (uint32_t)s * 2 * kLBO, kLBO, kSBO), idesc, 1u);
 }
 
 template <int MODE, bool SPLIT>
@@ -314,10 +332,10 @@ lse_tmem_kernel(const float* __restrict__ src, const float* __restrict__ src2, c
             if (lane == 0) {
                 if (ok) {
                     const uint32_t idesc = idesc_n(n_pad);
-                    const uint32_t w = smem_u32(sm), wl = w + (uint32_t)n_pad * KT * 2;
+                    const uint32_t w = smem_u32(sm), wp = (uint32_t)n_pad * KT * 2;
                     const uint32_t a = taddr + kColsD;
                     const int steps = (terms_of(i) + 15) / 16;
-                    issue_mmas<SPLIT>(taddr, a, w, wl, steps, idesc, nch_tile > 1);
+                    issue_mmas<SPLIT ? 2 : 1>(taddr, a, w, wp, steps, idesc, nch_tile > 1);
                 } else {
                     slot[1] = 1;
                 }
@@ -602,6 +620,13 @@ lse_tmem_kernel(const float* __restrict__ src, const float* __restrict__ src2, c
 // chunks keeps both accumulators apart until its end; of more, the older one goes to FP32 sums
 // in shared memory (for the same reason as above). Consecutive slices of a tile reuse its
 // weights.
+//
+// NP parts per operand: 1 single bf16, 2 split (hi, lo), 3 for the plain FP32 form (hi, mid, lo:
+// 24 bits; the six products down to 2^-18, smallest first, then hi * hi alone truncates). With
+// three parts A has one slot, D's two hold one chunk, whose sums go to shared memory when another
+// follows, and the weights then have one slot too. 119 tiles of 128 x
+// 128, batch 512, FP32: 47 us with the pack against 102 us for FFMA; error against FP64 no larger (element flows 3.04e-7
+// against 3.06e-7).
 constexpr int kPWarps = 16;
 constexpr int kPThreads = 32 * kPWarps + 32;
 constexpr int PT = KT / 4;  // terms per thread and chunk
@@ -609,11 +634,13 @@ constexpr int EB = 8;       // accumulator columns per epilogue step
 constexpr int kRowRing = 4;
 
 struct PSmem {
-    uint32_t sum, part, rows, bar, slot, total;  // two weight slots come first
-    __host__ __device__ PSmem(int n_pad, bool sums) {
-        const uint32_t w = (uint32_t)n_pad * KT * 4;
-        sum = 2 * w;
-        part = sum + (sums ? w : 0);        // [2 buffers][4 parts][NS] chunk maxima
+    uint32_t wslot, sum, part, rows, bar, slot, total;  // the weight slots come first
+    int nw;
+    __host__ __device__ PSmem(int n_pad, int np, bool sums) {
+        wslot = (uint32_t)n_pad * KT * 2 * (np < 2 ? 2 : np);
+        nw = np == 3 && sums ? 1 : 2;
+        sum = nw * wslot;
+        part = sum + (sums ? (uint32_t)n_pad * NS * 4 : 0);  // [2 buffers][4 parts][NS] chunk maxima
         rows = part + 2 * 4 * NS * 4;       // [kRowRing][KT]
         bar = rows + kRowRing * KT * 4;
         slot = bar + 16 * 8;
@@ -633,7 +660,7 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&v)[8]) {
 // exp(m - to) for a scale between maxima; equal ones (also both -inf) give 1
 __device__ __forceinline__ float rescale(float m, float to) { return m == to ? 1.f : pcb::fast_exp(m - to); }
 
-template <int MODE, bool SPLIT>
+template <int MODE, int NP>
 __global__ void __launch_bounds__(kPThreads, 1)
 lse_tmem_persistent_kernel(const float* __restrict__ src, const float* __restrict__ src2,
                            const float* __restrict__ aux, float* __restrict__ out, int64_t ld, int B,
@@ -642,8 +669,9 @@ lse_tmem_persistent_kernel(const float* __restrict__ src, const float* __restric
                            bool sums, int num_slices, int num_units, int32_t* __restrict__ status) {
     pcb::pdl_trigger();
     extern __shared__ __align__(1024) uint8_t sm[];
-    const PSmem S(n_max, sums);
-    const uint32_t wslot = (uint32_t)n_max * KT * 4;
+    constexpr int AS = NP == 3 ? 1 : 2;  // slots of A
+    static_assert(NP < 3 || MODE < 2, "the FP32 form takes rewritten flows");
+    const PSmem S(n_max, NP, sums);
     float* sSum = reinterpret_cast<float*>(sm + S.sum);  // [rows][samples]
     float* sPart = reinterpret_cast<float*>(sm + S.part);
     int* sRows = reinterpret_cast<int*>(sm + S.rows);
@@ -673,9 +701,9 @@ lse_tmem_persistent_kernel(const float* __restrict__ src, const float* __restric
     __syncthreads();
     fence_after_sync();
     const uint32_t taddr = slot[0];
-    // columns: D of slots 0 and 1, then A (hi, lo) of slots 0 and 1
-    auto d_cols = [&](int q) { return taddr + (q & 1) * kColsD; };
-    auto a_cols = [&](int q) { return taddr + 2 * kColsD + (q & 1) * 2 * kColsA; };
+    // columns: D of slots 0 and 1, then A (its parts side by side) of slots 0 and 1
+    auto d_cols = [&](int q) { return taddr + (NP == 3 ? 0 : (q & 1) * kColsD); };
+    auto a_cols = [&](int q) { return taddr + 2 * kColsD + (AS == 1 ? 0 : (q & 1) * 2 * kColsA); };
     auto chunks_of = [&](const PcbLseTile& t) { return max(1, (t.k_cnt + KT - 1) / KT); };
     bool fail = false;
 
@@ -702,16 +730,16 @@ lse_tmem_persistent_kernel(const float* __restrict__ src, const float* __restric
             const int tile_id = wu / num_slices;
             const PcbLseTile t = tiles[tile_id];
             const int c = chunk_index ? __ldg(chunk_index + (int64_t)tile_id * chunk_ld + wi) : tile_id;
-            const int sl = wq & 1;
+            const int sl = S.nw == 1 ? 0 : wq & 1;
             if (held[sl] != c) {
                 held[sl] = c;
                 ++loads[sl];
                 if (lane == 0) {
-                    const uint8_t* w = packed + (size_t)c * kTileBytes;
-                    const uint32_t half = (uint32_t)((t.n_rows + 15) & ~15) * KT * 2;
-                    mbar_expect_tx(barW + sl, SPLIT ? 2 * half : half);
-                    bulk_copy_g2s(sm + sl * wslot, w, half, barW + sl);
-                    if (SPLIT) bulk_copy_g2s(sm + sl * wslot + half, w + kHalfBytes, half, barW + sl);
+                    const uint8_t* w = packed + (size_t)c * (NP == 3 ? 3 * kHalfBytes : kTileBytes);
+                    const uint32_t bytes = (uint32_t)((t.n_rows + 15) & ~15) * KT * 2;
+                    mbar_expect_tx(barW + sl, NP * bytes);
+                    for (int p = 0; p < NP; ++p)
+                        bulk_copy_g2s(sm + sl * S.wslot + p * bytes, w + p * kHalfBytes, bytes, barW + sl);
                 }
             }
             ++wq;
@@ -721,7 +749,7 @@ lse_tmem_persistent_kernel(const float* __restrict__ src, const float* __restric
         put_rows();
         put_rows();
         pcb::pdl_wait();
-        copy_weights();
+        if (S.nw == 2) copy_weights();
         int q = 0;
         for (int u = u0; u < u1; ++u) {
             const PcbLseTile t = tiles[u / num_slices];
@@ -729,19 +757,21 @@ lse_tmem_persistent_kernel(const float* __restrict__ src, const float* __restric
             const int n_pad = (t.n_rows + 15) & ~15;
             for (int i = 0; i < nch; ++i, ++q) {
                 const int sl = q & 1;
-                // chunk q + 1's weights once the MMAs of chunk q - 1 have left their slot
+                // chunk q + 1's weights (with one slot chunk q's) once the MMAs of chunk q - 1 have
+                // left their slot
                 if (q > 0 && !mbar_wait_bounded(barM + (sl ^ 1), (uint32_t)(((q - 1) >> 1) & 1)) && lane == 0) slot[1] = 1;
                 copy_weights();
                 bool ok = mbar_wait_bounded(barA + sl, (uint32_t)((q >> 1) & 1));
-                ok = mbar_wait_bounded(barW + sl, (uint32_t)((loads[sl] - 1) & 1)) && ok;
+                const int ws = S.nw == 1 ? 0 : sl;
+                ok = mbar_wait_bounded(barW + ws, (uint32_t)((loads[ws] - 1) & 1)) && ok;
                 fence_after_sync();
                 if (lane == 0) {
                     if (ok) {
                         const uint32_t idesc = idesc_n(n_pad);
-                        const uint32_t w = smem_u32(sm + sl * wslot), wl = w + (uint32_t)n_pad * KT * 2;
+                        const uint32_t w = smem_u32(sm + ws * S.wslot), wp = (uint32_t)n_pad * KT * 2;
                         const uint32_t a = a_cols(q), d = d_cols(q);
                         const int steps = max(1, (min(KT, t.k_cnt - i * KT) + 15) / 16);
-                        issue_mmas<SPLIT>(d, a, w, wl, steps, idesc, nch > 1);
+                        issue_mmas<NP>(d, a, w, wp, steps, idesc, nch > 1);
                     } else {
                         slot[1] = 1;
                     }
@@ -803,7 +833,7 @@ lse_tmem_persistent_kernel(const float* __restrict__ src, const float* __restric
             fail = fail || slot[1] != 0;
             const bool in = b0 + s < B, active = b0 + (warp & 3) * 32 < B;
             const int blocks = ((t.n_rows + 15) & ~15) / EB;
-            const float f1 = nch > 1 ? rescale(m1, m0) : 0.f, fs = nch > 2 ? rescale(ms, m0) : 0.f;
+            const float f1 = nch > 1 ? rescale(m1, m0) : 0.f, fs = nch > (NP == 3 ? 1 : 2) ? rescale(ms, m0) : 0.f;
             const float* ax = MODE != 0 ? aux + (int64_t)t.aux_row * ld + min(b0 + s, B - 1) : nullptr;
             float* o = out + (int64_t)t.out_row * ld + b0 + s;
             float a[MODE == 0 ? 1 : EB];
@@ -819,7 +849,17 @@ lse_tmem_persistent_kernel(const float* __restrict__ src, const float* __restric
             for (int blk = part; blk < blocks; blk += 4) {
                 float d[EB];
                 tmem_ld8(d_cols(q) + tlane + blk * EB, d);
-                if (nch > 1) {
+                if (NP == 3) {
+                    float e[EB];
+                    tmem_ld8(d_cols(q) + kColsD + tlane + blk * EB, e);
+                    wait_ld();
+#pragma unroll
+                    for (int j = 0; j < EB; ++j) d[j] += e[j];
+                    if (nch > 1) {
+#pragma unroll
+                        for (int j = 0; j < EB; ++j) d[j] = fmaf(sSum[(blk * EB + j) * NS + s], fs, d[j]);
+                    }
+                } else if (nch > 1) {
                     float e[EB];
                     tmem_ld8(d_cols(q - 1) + tlane + blk * EB, e);
                     wait_ld();
@@ -832,7 +872,10 @@ lse_tmem_persistent_kernel(const float* __restrict__ src, const float* __restric
                 } else {
                     wait_ld();
                 }
-                if (MODE == 0) {
+                if (MODE == 0 && NP == 3) {
+#pragma unroll
+                    for (int j = 0; j < EB; ++j) d[j] = m0 == -INFINITY ? -INFINITY : logf(d[j]) + m0;
+                } else if (MODE == 0) {
                     float m[EB];
 #pragma unroll
                     for (int j = 0; j < EB; ++j) m[j] = m0;
@@ -893,29 +936,30 @@ lse_tmem_persistent_kernel(const float* __restrict__ src, const float* __restric
                 asm volatile("bar.sync 1, 512;\n" ::: "memory");
                 m = fmaxf(fmaxf(fmaxf(pm[0], pm[NS]), fmaxf(pm[2 * NS], pm[3 * NS])), mrun);
                 mrun = m;
-                // A's slot: the MMAs of chunk q - 2 have read it
-                if (q >= 2 && !mbar_wait_bounded(barM + (q & 1), (uint32_t)(((q - 2) >> 1) & 1))) fail = true;
+                // A's slot: the MMAs of chunk q - AS have read it
+                if (q >= AS && !mbar_wait_bounded(barM + ((q - AS) & 1), (uint32_t)(((q - AS) >> 1) & 1))) fail = true;
                 fence_after_sync();
                 const float mu = m == -INFINITY ? 0.f : m;
                 const uint64_t nmu = pair(-mu, -mu);
                 const uint32_t ta = a_cols(q) + tlane + part * (PT / 2);
 #pragma unroll
                 for (int g = 0; g < PT; g += 16) {
-                    uint32_t hi[8], lo[8];
+                    uint32_t parts[NP][8];
 #pragma unroll
                     for (int j = 0; j < 8; ++j) {
                         const uint64_t x = mul2(add2(pair(v[g + 2 * j], v[g + 2 * j + 1]), nmu), log2e);
                         const float2 x2 = unpair(x);
-                        const float e0 = ex2(x2.x), e1 = ex2(x2.y);
-                        hi[j] = bf16x2(e0, e1);
-                        if (SPLIT) {
-                            const uint64_t h = pair(__uint_as_float(hi[j] << 16), __uint_as_float(hi[j] & 0xffff0000u));
-                            const float2 l = unpair(fma2(h, minus1, pair(e0, e1)));
-                            lo[j] = bf16x2(l.x, l.y);
+                        uint64_t e = pair(ex2(x2.x), ex2(x2.y));
+#pragma unroll
+                        for (int p = 0; p < NP; ++p) {
+                            const float2 f = unpair(e);
+                            const uint32_t h = parts[p][j] = bf16x2(f.x, f.y);
+                            if (p + 1 < NP)
+                                e = fma2(pair(__uint_as_float(h << 16), __uint_as_float(h & 0xffff0000u)), minus1, e);
                         }
                     }
-                    tmem_st8(ta + g / 2, hi);
-                    if (SPLIT) tmem_st8(ta + kColsA + g / 2, lo);
+#pragma unroll
+                    for (int p = 0; p < NP; ++p) tmem_st8(ta + p * kColsA + g / 2, parts[p]);
                 }
                 // the next chunk's rows
                 const bool last = i + 1 == nch;
@@ -926,21 +970,25 @@ lse_tmem_persistent_kernel(const float* __restrict__ src, const float* __restric
                 // D's slot: what chunk q - 2 left there
                 if (i == 0) {
                     if (u > u0) finish(q - 1, tp, nchp, b0p);
-                } else if (i >= 2) {
-                    const float f = i > 2 ? rescale(ms, m1) : 0.f;
+                } else if (i >= (NP == 3 ? 1 : 2)) {
+                    const float mo = NP == 3 ? m0 : m1;  // what that accumulator is relative to
+                    const bool more = i > (NP == 3 ? 1 : 2);
+                    const float f = more ? rescale(ms, mo) : 0.f;
                     const int blocks = ((t.n_rows + 15) & ~15) / EB;
 #pragma unroll 1
                     for (int blk = part; blk < blocks; blk += 4) {
-                        float d[EB];
+                        float d[EB], e[EB];
                         tmem_ld8(d_cols(q) + tlane + blk * EB, d);
+                        if (NP == 3) tmem_ld8(d_cols(q) + kColsD + tlane + blk * EB, e);
                         wait_ld();
 #pragma unroll
                         for (int j = 0; j < EB; ++j) {
                             float* p = sSum + (blk * EB + j) * NS + s;
-                            *p = i > 2 ? fmaf(*p, f, d[j]) : d[j];
+                            const float x = NP == 3 ? d[j] + e[j] : d[j];
+                            *p = more ? fmaf(*p, f, x) : x;
                         }
                     }
-                    ms = m1;
+                    ms = mo;
                 }
                 m1 = m0;
                 m0 = m;
@@ -964,19 +1012,19 @@ lse_tmem_persistent_kernel(const float* __restrict__ src, const float* __restric
     }
 }
 
-template <int MODE, bool SPLIT>
+template <int MODE, int NP>
 int launch_persistent(const float* src, const float* src2, const float* aux, float* out, int64_t ld, int B,
                       const uint8_t* packed, const PcbLseTile* tiles, int num_tiles, int n_max, const int* krow,
                       const int* chunk_index, int chunk_ld, cudaStream_t s) {
-    const bool sums = chunk_index && chunk_ld > 2;
-    const size_t smem = PSmem(n_max, sums).total;
+    const bool sums = chunk_index && chunk_ld > (NP == 3 ? 1 : 2);
+    const size_t smem = PSmem(n_max, NP, sums).total;
     static bool configured[64] = {false};
     static int sms[64] = {0};
     int dev = 0;
     cudaGetDevice(&dev);
     dev = dev < 0 ? 0 : (dev > 63 ? 63 : dev);
     if (!configured[dev]) {
-        cudaError_t e = cudaFuncSetAttribute(lse_tmem_persistent_kernel<MODE, SPLIT>,
+        cudaError_t e = cudaFuncSetAttribute(lse_tmem_persistent_kernel<MODE, NP>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
         if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms[dev], cudaDevAttrMultiProcessorCount, dev);
         if (e != cudaSuccess) return pcb::set_error(PCB_E_CUDA, "pcb_lse_contract_tmem: %s", cudaGetErrorString(e));
@@ -986,7 +1034,7 @@ int launch_persistent(const float* src, const float* src2, const float* aux, flo
     const int64_t units = (int64_t)num_tiles * slices;
     if (units > INT32_MAX) return pcb::set_error(PCB_E_ARG, "pcb_lse_contract_tmem: too many tiles");
     return pcb::launch_status(
-        pcb::launch_k(lse_tmem_persistent_kernel<MODE, SPLIT>, dim3((unsigned)std::min<int64_t>(units, sms[dev])),
+        pcb::launch_k(lse_tmem_persistent_kernel<MODE, NP>, dim3((unsigned)std::min<int64_t>(units, sms[dev])),
                       dim3(kPThreads), smem, s, 1u, src, src2, aux, out, ld, B, packed, tiles, krow, chunk_index,
                       chunk_ld, n_max, sums, slices, (int)units, pcb::status_word()),
         "pcb_lse_contract_tmem");
@@ -1027,7 +1075,8 @@ extern "C" int pcb_lse_contract_tmem(const float* src, const float* src2, const 
                                      int32_t tile_rows, const int32_t* krow, const int32_t* chunk_index,
                                      int32_t chunk_ld, int32_t mode, int32_t prec, int32_t ksplit, void* stream) {
     if (!src || !out || !packed || !tiles || !krow || B <= 0 || ld < B || num_tiles < 0 || tile_rows < 1 ||
-        tile_rows > 128 || mode < 0 || mode > 2 || (mode == 2 && !src2) || (mode >= 1 && !aux) || prec < 1 || prec > 2 ||
+        tile_rows > 128 || mode < 0 || mode > 2 || (mode == 2 && !src2) || (mode >= 1 && !aux) || prec < 0 || prec > 2 ||
+        (prec == 0 && (ksplit != 0 || mode == 2)) ||
         ksplit < 0 || ksplit > kMaxCluster || (chunk_index && chunk_ld < 1) ||
         (reinterpret_cast<uintptr_t>(packed) & 15) != 0)
         return pcb::set_error(PCB_E_ARG, "pcb_lse_contract_tmem: bad arguments");
@@ -1035,12 +1084,11 @@ extern "C" int pcb_lse_contract_tmem(const float* src, const float* src2, const 
     const int n_max = (tile_rows + 15) & ~15;
     cudaStream_t s = pcb::as_stream(stream);
     if (ksplit == 0) {
-#define PCB_TP(M) \
-    (prec == 2 ? launch_persistent<M, true>(src, src2, aux, out, ld, B, packed, tiles, num_tiles, n_max, krow, \
-                                            chunk_index, chunk_ld, s) \
-               : launch_persistent<M, false>(src, src2, aux, out, ld, B, packed, tiles, num_tiles, n_max, krow, \
-                                             chunk_index, chunk_ld, s))
-        return mode == 0 ? PCB_TP(0) : (mode == 1 ? PCB_TP(1) : PCB_TP(2));
+#define PCB_TP(M, P) \
+    launch_persistent<M, P>(src, src2, aux, out, ld, B, packed, tiles, num_tiles, n_max, krow, chunk_index, chunk_ld, s)
+        if (prec == 0) return mode == 0 ? PCB_TP(0, 3) : PCB_TP(1, 3);
+        if (prec == 1) return mode == 0 ? PCB_TP(0, 1) : (mode == 1 ? PCB_TP(1, 1) : PCB_TP(2, 1));
+        return mode == 0 ? PCB_TP(0, 2) : (mode == 1 ? PCB_TP(1, 2) : PCB_TP(2, 2));
 #undef PCB_TP
     }
 #define PCB_TM(M) \

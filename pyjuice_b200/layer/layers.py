@@ -131,6 +131,18 @@ def _chunk_index(tiles_np: np.ndarray) -> np.ndarray:
     return index
 
 
+_PACK3_BYTES = 98304  # the same weights in three bf16 parts (pcb_pack_weights_f32)
+
+
+def _pack3(holder: dict, table: torch.Tensor) -> torch.Tensor:
+    """The three-part packs of a tile or chunk table (FP32 form), allocated on the device at first
+    use; tied layers hold one buffer (``holder["pack3_of"]``, set by the circuit)."""
+    h = holder.get("pack3_of") or holder
+    if h.get("pack3") is None:
+        h["pack3"] = torch.empty([table.size(0) * _PACK3_BYTES], dtype=torch.uint8, device=table.device)
+    return h["pack3"]
+
+
 def _tmem_ksplit(num_tiles: int, tile_rows: int, num_chunks: int, B: int) -> int:
     """CTAs (a cluster) that share a tile's chunks in pcb_lse_contract_tmem (``ksplit``). Tiles
     of more than 64 rows: one per chunk, so that two CTAs fit on an SM (the sums of several
@@ -682,7 +694,7 @@ class SumLayer(Layer):
                 ch_pack=None, ch_pack_bytes=0 if ech_t is None else ech_t[0].shape[0] * _PACK_BYTES,
                 cbs=cbs, tm=_tile_rows(max(t[1] for t in tiles)), tiles=_i32(tiles_np),
                 krow=_i32(np.concatenate(klist)), kw=_i32(kw_np),
-                short=int(tiles_np[:, 3].max()) <= _SHORT_K,
+                short=int(tiles_np[:, 3].max()) <= _SHORT_K, max_terms=int(tiles_np[:, 3].max()),
                 wlayout=2 if _terms_vec4(tiles_np, kw_np, bs) else 0,
                 run=_run_rows(tiles_np, np.concatenate(klist)),
                 pack=torch.empty([tiles_np.shape[0] * _PACK_BYTES], dtype=torch.uint8)))
@@ -692,6 +704,7 @@ class SumLayer(Layer):
         return dict(
             fw_ch=None if fch is None else _i32(fch[0]), fw_ch_ranges=None if fch is None else fch[1],
             fw_ch_index=None if fch is None else _i32(_chunk_index(fw_np)),
+            fw_f32=dict(pack3=None), fw_max_terms=int(fw_np[:, 3].max()) if fw_np.shape[0] else 0,
             fw_ch_pack=None, fw_ch_pack_bytes=0 if fch is None else fch[0].shape[0] * _PACK_BYTES,
             fw_tiles=_i32(fw_np), fw_tm=fw_tm, fw_run=_run_rows(fw_np, krow_c),
             fw_short=bool(fw_np.shape[0]) and int(fw_np[:, 3].max()) <= _SHORT_K,
@@ -759,6 +772,30 @@ class SumLayer(Layer):
         return (prec > 0 and SumLayer.tc05_long and not eg["short"] and eg["ch"] is not None
                 and eg["ch"].size(0) >= SumLayer.tc05_min_tiles)
 
+    @staticmethod
+    def _f32_tmem(tiles, tile_rows, max_terms, table, B):
+        """Whether an FP32 contraction runs on the tensor cores in three bf16 parts (the persistent
+        pcb_lse_contract_tmem): tiles of at least 64 rows and terms, and a (tile, 128-sample
+        slice) for every other SM. Measured, forward with the pack against FFMA (us, batch 512):
+        200 regions of 256 x 256: 197 / 773; 119 of 128 x 128: 47 / 102; 40 of 64 x 512: 48 / 84; 25
+        of 96 x 96: 12.7 / 18.6; 100 of 32 x 32: 18.7 / 13.1."""
+        return (SumLayer.tmem is not False and SumLayer.tc05_long and tile_rows >= 64 and max_terms >= 64
+                and table is not None and tiles.size(0) >= SumLayer.tc05_min_tiles
+                and 2 * tiles.size(0) * -(-B // 128) >= _num_sms())
+
+    def _fw_f32(self, d, B):
+        return self._f32_tmem(d["fw_tiles"], d["fw_tm"], d["fw_max_terms"],
+                              d["fw_tiles"] if d["fw_short"] else d["fw_ch"], B)
+
+    def _el_f32(self, eg, B):
+        return self._f32_tmem(eg["tiles"], eg["tm"], eg["max_terms"], eg["tiles"] if eg["short"] else eg["ch"], B)
+
+    @staticmethod
+    def _run_f32(holder, tiles, tile_rows, table, index, src, aux, out, ld, B, krow, mode):
+        nat.call("pcb_lse_contract_tmem", nat.ptr(src), nat.ptr(None), nat.ptr(aux), nat.ptr(out), ld, B,
+                 nat.ptr(_pack3(holder, table)), nat.ptr(tiles), tiles.size(0), tile_rows, nat.ptr(krow),
+                 nat.ptr(index), 0 if index is None else index.size(1), mode, 0, 0, nat.stream())
+
     def _el_tc05(self, eg, prec):
         return prec > 0 and eg["short"] and eg["tiles"].size(0) >= SumLayer.tc05_min_tiles
 
@@ -770,7 +807,9 @@ class SumLayer(Layer):
         if not SumLayer.short_kernels:
             return False
         if not backward:
-            return d["fw_short"] and not self._fw_tc05(d, B, force_use_bf16, force_use_fp32)[1]
+            prec, tc05 = self._fw_tc05(d, B, force_use_bf16, force_use_fp32)
+            return d["fw_short"] and not tc05 and not (prec == 0 and self._fw_f32(d, B))
+        # (the FP32 form on the tensor cores takes rewritten flows, which are never fused)
         return all(eg["short"] and not self._el_tc05(eg, self._el_prec(eg, B, force_use_fp32))
                    for eg in d["el_groups"])
 
@@ -785,6 +824,9 @@ class SumLayer(Layer):
             return (d["fw_tiles"], d["kw"], d["fw_pack"], self.block_size, 1, 1 if (tc05 and prec == 3) else 0)
         if self._fw_long(d, prec):
             return (d["fw_ch"], d["kw"], _ch_pack(d, "fw_ch_pack"), self.block_size, 1, 1 if prec == 3 else 0)
+        if prec == 0 and self._fw_f32(d, B):
+            table = d["fw_tiles"] if d["fw_short"] else d["fw_ch"]
+            return (table, d["kw"], _pack3(d["fw_f32"], table), self.block_size, 1, 2)
         return None
 
     def flow_pack_jobs(self, device: torch.device, B: int, force_use_fp32: bool = False):
@@ -799,12 +841,15 @@ class SumLayer(Layer):
                              1 if (tc05 and prec == 3) else 0))
             elif self._el_long(eg, prec):
                 jobs.append((eg["ch"], eg["kw"], _ch_pack(eg, "ch_pack"), eg["cbs"], self.block_size, 1 if prec == 3 else 0))
+            elif prec == 0 and self._el_f32(eg, B):
+                table = eg["tiles"] if eg["short"] else eg["ch"]
+                jobs.append((table, eg["kw"], _pack3(eg, table), eg["cbs"], self.block_size, 2))
         return jobs
 
     @staticmethod
     def _run_pack_job(params: torch.Tensor, job) -> None:
         t, kw, packed, rpb, w_stride, fmt = job
-        nat.call("pcb_pack_weights_fp8" if fmt == 1 else "pcb_pack_weights", nat.ptr(params), nat.ptr(t), t.size(0),
+        nat.call(("pcb_pack_weights", "pcb_pack_weights_fp8", "pcb_pack_weights_f32")[fmt], nat.ptr(params), nat.ptr(t), t.size(0),
                  rpb, nat.ptr(kw), w_stride, nat.ptr(packed), nat.stream())
 
     def pack_forward_weights(self, params: torch.Tensor, B: int, force_use_bf16: bool = False,
@@ -889,6 +934,13 @@ class SumLayer(Layer):
                        d["fw_ch_ranges"], d["krow"], 0, prec, st, holder=d, plan_key="fw_ch_plan", tiles=t,
                        tile_rows=d["fw_tm"], index=d["fw_ch_index"])
             return
+        if prec == 0 and kwargs.get("_fuse_fw") is None and self._fw_f32(d, B):
+            if not _weights_packed:
+                self.pack_forward_weights(params, B, force_use_bf16, force_use_fp32)
+            short = d["fw_short"]
+            self._run_f32(d["fw_f32"], t, d["fw_tm"], t if short else d["fw_ch"], None if short else d["fw_ch_index"],
+                          element_mars, None, node_mars, ld, B, d["krow"], 0)
+            return
         prec = _mma(prec)
         # _fuse_fw = (term_children, element values out): the product layer below is fused in
         # (the terms are sums of node rows; the element values are written as a side output)
@@ -946,11 +998,15 @@ class SumLayer(Layer):
             nat.call("pcb_modify_flows", nat.ptr(node_flows), nat.ptr(node_mars), ld, B, self._layer_nid_range[0],
                      self._layer_nid_range[1], nat.stream())
         flows, modified = node_flows, allow_modify_flows
+
+        def packed_form(eg):  # runs on the kernels that read packed weights
+            p = self._el_prec(eg, B, force_use_fp32)
+            return self._el_tc05(eg, p) or self._el_long(eg, p) or (p == 0 and self._el_f32(eg, B))
+
         if (not allow_modify_flows and kwargs.get("_pflow_stream") is None and kwargs.get("_fuse_bw") is None
-                and not force_use_fp32 and SumLayer.bf16_form != 3
+                and (force_use_fp32 or SumLayer.bf16_form != 3)
                 and (self._layer_nid_range[1] - self._layer_nid_range[0]) * B >= SumLayer.ratio_min_values
-                and all(self._el_tc05(eg, p) or self._el_long(eg, p)
-                                                    for eg in d["el_groups"] for p in (self._el_prec(eg, B, False),))):
+                and all(map(packed_form, d["el_groups"]))):
             # log f - log m of this layer's nodes once, in a workspace, instead of in every tile
             # of both contractions that reads them (node_flows stays as the caller has it)
             lo, hi = self._layer_nid_range
@@ -970,7 +1026,8 @@ class SumLayer(Layer):
             ready = torch.cuda.Event()
             ready.record()
         # element flows
-        if not _weights_packed and any(self._el_tc05(eg, p) or self._el_long(eg, p)
+        if not _weights_packed and any(self._el_tc05(eg, p) or self._el_long(eg, p) or
+                                       (p == 0 and modified and self._el_f32(eg, B))
                                        for eg in d["el_groups"] for p in (self._el_prec(eg, B, force_use_fp32),)):
             self.pack_flow_weights(params, B, force_use_fp32)
             _weights_packed = True
@@ -987,6 +1044,11 @@ class SumLayer(Layer):
                            _ch_pack(eg, "ch_pack"), eg["ch"], eg["ch_ranges"], eg["krow"], 1 if modified else 2,
                            prec, nat.stream(), holder=eg, plan_key="ch_plan", tiles=et, tile_rows=eg["tm"],
                            index=eg["ch_index"])
+                continue
+            if prec == 0 and modified and self._el_f32(eg, B):
+                short = eg["short"]
+                self._run_f32(eg, et, eg["tm"], et if short else eg["ch"], None if short else eg["ch_index"], flows,
+                              element_mars, element_flows, ld, B, eg["krow"], 1)
                 continue
             prec = _mma(prec)
             if eg["short"] and SumLayer.short_kernels:

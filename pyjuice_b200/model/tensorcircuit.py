@@ -618,11 +618,20 @@ class TensorCircuit(nn.Module):
             fh, fk, flazy = first
             holder[pack_key] = _ch_pack(fh, fk) if flazy else fh[fk]
 
+        def share3(role, holder, table, rpb, w_stride, kw):  # the FP32 form's packs, made on demand
+            c = None if table is None else content(table, kw)
+            if c is not None:
+                first = canon.setdefault((role, rpb, w_stride) + c, holder)
+                holder["pack3_of"] = None if first is holder else first
+
         for group in self.inner_layer_groups:
             if not group.is_sum():
                 continue
             for layer in group:
                 d = layer._desc(self.device)
+                share3("fw3", d["fw_f32"], d["fw_tiles"] if d["fw_short"] else d["fw_ch"], layer.block_size, 1, d["kw"])
+                for eg in d["el_groups"]:
+                    share3("el3", eg, eg["tiles"] if eg["short"] else eg["ch"], eg["cbs"], layer.block_size, eg["kw"])
                 share("fw", d, "fw_tiles", "fw_pack", layer.block_size, 1, d["kw"], False)
                 share("fwch", d, "fw_ch", "fw_ch_pack", layer.block_size, 1, d["kw"], True)
                 for eg in d["el_groups"]:
@@ -715,7 +724,7 @@ class TensorCircuit(nn.Module):
         """What the element-flow packs depend on: the parameter values (storage, torch version
         counter, in-library writes) and the settings that select the packed layers."""
         return (self.params.data_ptr(), self.params._version, self._param_epoch, B, bool(force_use_fp32),
-                SumLayer.bf16_form, SumLayer.pack_short_weights, SumLayer.tc05_min_tiles)
+                SumLayer.bf16_form, SumLayer.pack_short_weights, SumLayer.tc05_min_tiles, SumLayer.tmem is not False)
 
     # The forward of the run of small levels next to the root (product layer fused into the
     # single-stage sum kernel above it) in one persistent launch (pcb_lse_levels_short)

@@ -86,6 +86,51 @@ def test_contractions(regions, nodes, terms, bs, B, ksplit, form, cuda_device, s
     assert nat.device_status() == 0
 
 
+@pytest.mark.parametrize("regions,nodes,terms,bs,B", [(1, 64, 64, 32, 1), (2, 128, 128, 32, 129), (3, 80, 112, 16, 300),
+                                                      (2, 128, 144, 16, 127), (1, 64, 400, 16, 260), (40, 128, 256, 32, 512)])
+def test_fp32_form(regions, nodes, terms, bs, B, cuda_device, settings, monkeypatch):
+    """The plain FP32 form on three-part operands: values and element flows against FP64."""
+    from pyjuice_b200.layer import layers as mod
+    SumLayer.tc05_min_tiles, SumLayer.ratio_min_values = 1, 0
+    monkeypatch.setattr(mod, "_num_sms", lambda: 1)
+    layer = _layer(regions, nodes, terms, bs, cuda_device)
+    d = layer._desc(torch.device(cuda_device))
+    assert layer._fw_f32(d, B) and all(layer._el_f32(eg, B) for eg in d["el_groups"])
+    gen = torch.Generator(device=cuda_device).manual_seed(nodes + terms + B)
+    rnd = lambda *shape: torch.rand(shape, generator=gen, device=cuda_device)
+    w = torch.exp(-4.0 * rnd(regions, nodes, terms))
+    w = w / w.sum(dim=2, keepdim=True)
+    params = torch.cat([torch.zeros([bs ** 2], device=cuda_device),
+                        w.reshape(regions, nodes // bs, bs, terms).permute(0, 1, 3, 2).reshape(-1)])
+    em = -12.0 * rnd(regions, terms, B)
+    em[rnd(regions, terms, B) < 0.1] = -float("inf")
+    em[0, :, 0] = -float("inf")
+    ems = torch.cat([torch.full([bs, B], -float("inf"), device=cuda_device), em.reshape(-1, B)])
+    nm = torch.full([bs + regions * nodes, B], 5.0, device=cuda_device)
+    layer(nm, ems, params, force_use_fp32=True)
+    ref = torch.log(w.double() @ em.double().exp())
+    got = nm[bs:].reshape(regions, nodes, B).double()
+    assert torch.equal(torch.isinf(got), torch.isinf(ref))
+    fin = torch.isfinite(ref)
+    # exponents of magnitude up to 18 rounded twice (2 * 18 * 2^-24), the exponential's 2^-21, 10
+    # truncations of 2^-23, the logarithm and the sum with the maximum 2 * 2^-24 of the value
+    assert torch.all((got - ref)[fin].abs() <= 4e-6 + 2.0 ** -22 * ref[fin].abs())
+    nms = torch.cat([torch.zeros([bs, B], device=cuda_device), ref.float().reshape(-1, B)])
+    nf = torch.softmax(3.0 * rnd(regions, nodes, B), dim=1)
+    nf[rnd(regions, nodes, B) < 0.1] = 0.0
+    nfs = torch.cat([torch.zeros([bs, B], device=cuda_device), nf.reshape(-1, B)])
+    nm64 = ref.float().double()
+    ratio = torch.where(torch.isfinite(nm64), nf.double() * torch.exp(-nm64), 0.0)
+    want = (w.double().transpose(1, 2) @ ratio) * em.double().exp()
+    for modify in (False, True):
+        ef = torch.full_like(ems, 9.0)
+        layer.backward(nfs.clone(), ef, nms, ems, params, None, allow_modify_flows=modify, force_use_fp32=True)
+        # as above with four roundings of exponents of magnitude up to 30
+        assert torch.all((ef[bs:].reshape(regions, terms, B).double() - want).abs() <= 1.2e-5 * want)
+        assert torch.all(ef[:bs] == 9.0)
+    assert nat.device_status() == 0
+
+
 @pytest.mark.parametrize("nodes,terms,bs,B,form", [(16, 16, 16, 1, 2), (128, 64, 32, 64, 2), (144, 80, 16, 65, 2), (256, 256, 32, 257, 2),
                                                    (48, 200, 8, 511, 2), (64, 128, 64, 130, 1)])
 @pytest.mark.parametrize("children", [64, 128])
