@@ -283,6 +283,8 @@ lse_tmem_kernel(const float* __restrict__ src, const float* __restrict__ src2, c
         tmem_alloc(slot, kCols);
         fence_before_sync();
     }
+    // the first chunk's source rows (compiled tables), the tile's first one beyond its terms
+    if (tid < KT && nch > 0) sRows[tid] = __ldg(krow + t.k_off + (tid < terms_of(0) ? chunk_of(0) * KT + tid : 0));
     if (tid == 0) {
         mbar_init(barW, 1);
         mbar_init(barM, 1);
@@ -299,20 +301,17 @@ lse_tmem_kernel(const float* __restrict__ src, const float* __restrict__ src2, c
     float own[2][16];  // this thread's sums of the column blocks that its CTA owns
 
     if (warp == 8) {
-        const int row0 = t.k_cnt > 0 ? __ldg(krow + t.k_off) : 0;
-        auto put_rows = [&](int i) {  // source rows of chunk i (compiled tables), the first one beyond its terms
+        auto put_rows = [&](int i) {  // source rows of a later chunk
             const int nk = terms_of(i);
-            const int* kr = krow + t.k_off + chunk_of(i) * KT;
             int* dst = sRows + (i & 1) * KT;
 #pragma unroll
             for (int j = 0; j < KT / 32; ++j) {
                 const int k = lane + 32 * j;
-                dst[k] = k < nk ? __ldg(kr + k) : row0;
+                dst[k] = __ldg(krow + t.k_off + (k < nk ? chunk_of(i) * KT + k : 0));
             }
             __syncwarp();
             if (lane == 0) mbar_arrive(barR + (i & 1));
         };
-        if (nch > 0) put_rows(0);
         if (nch > 1) put_rows(1);
         pcb::pdl_wait();
         auto copy_weights = [&](int i) {
@@ -366,7 +365,8 @@ lse_tmem_kernel(const float* __restrict__ src, const float* __restrict__ src2, c
         const uint32_t ta = tlane + kColsD + half * (HT / 2);      // hi, then lo
         const uint64_t log2e = pair(kLog2e, kLog2e), minus1 = pair(-1.f, -1.f);
         for (int i = 0; i < nch; ++i) {
-            if (!mbar_wait_bounded(barR + (i & 1), (uint32_t)((i >> 1) & 1))) fail = true;
+            // row numbers: buffer i & 1 is written for chunks 1, 3, .. and 2, 4, ..
+            if (i > 0 && !mbar_wait_bounded(barR + (i & 1), (uint32_t)(((i - 1) >> 1) & 1))) fail = true;
             const int4* rows = reinterpret_cast<const int4*>(sRows + (i & 1) * KT + half * HT);
             const int nk = terms_of(i) - half * HT;  // terms of this half
             if (i > 0) {
@@ -390,7 +390,7 @@ lse_tmem_kernel(const float* __restrict__ src, const float* __restrict__ src2, c
             }
             // values of the source rows: their maximum, and themselves to tensor memory
             float m = -INFINITY;
-            constexpr int G = MODE == 2 ? 16 : 32;  // rows in flight per thread (twice that in mode 2)
+            constexpr int G = MODE == 2 ? 32 : 64;  // rows whose loads are in flight together
 #pragma unroll 1
             for (int g = 0; g < HT; g += G) {
                 float v[G];

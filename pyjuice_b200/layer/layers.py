@@ -328,7 +328,7 @@ def _tc05_call(src, src2, aux, out, ld, B, pack, tiles, krow, mode, prec, stream
                      nat.ptr(pack), nat.ptr(tiles), nt, nat.ptr(krow), mode, prec, c[0], c[1], stream)
 
     shifted = isinstance(src, _ShiftedRows)
-    if prec != 3 and SumLayer.tmem not in (None, False):
+    if prec != 3 and SumLayer.tmem is not None and SumLayer.tmem is not False:
         return run(("tm", min(SumLayer.tmem, 1)))
     ws_ok = (not shifted and SumLayer.tc05_ws is not False and prec != 3 and run_rows in (8, 32)
              and _ws_ok(ld, B, src, src2, aux, out))
