@@ -26,9 +26,11 @@
 // that 16 chunks accumulated in D would be 1.3e-5 too small, against 3e-7 this way.
 //
 // Measured (forward, split form, weights packed, graph-timed): 119 tiles of 128 x 128, batch 512
-// (70 MB): 19.2 us, 3.7 TB/s, against 35.8 us for the best of the forms that keep the samples in
-// shared memory (lse_tc05.cu); 200 regions of 256 x 256 (262 MB): 87.5 us, 3.0 TB/s, on the
-// persistent form below, against 370 us in 128-term chunks. What is left: a chunk costs about
+// (70 MB): 18.1 us, 3.9 TB/s, against 35.9 us for the best of the forms that keep the samples in
+// shared memory (lse_tc05.cu); 200 regions of 256 x 256 (262 MB): 87.8 us, 3.0 TB/s, on the
+// persistent form below, against 315 us in 128-term chunks; element flows of the same layer
+// (367 MB): 113 us (139 us without the element values' prefetch), against
+// 452 us. What is left: a chunk costs about
 // 2,000 cycles of MMAs (three products), as many of exponentials, and its rows arrive at about
 // 20 bytes per SM and cycle.
 //
@@ -902,6 +904,15 @@ lse_tmem_persistent_kernel(const float* __restrict__ src, const float* __restric
             }
         };
 
+        // this warp's 128-byte lines of a unit's element values into L2, one line per lane, well
+        // ahead of finish()'s loads
+        auto prefetch_aux = [&](const PcbLseTile& t, int b0) {
+            const int r = (part + 4 * (lane / EB)) * EB + lane % EB;
+            const int b = b0 + (warp & 3) * 32;
+            if (r < t.n_rows && b < B)
+                asm volatile("prefetch.global.L2 [%0];\n" ::"l"(aux + ((int64_t)t.aux_row + r) * ld + b));
+        };
+
         using Z = std::integral_constant<int, 0>;
         using H = std::integral_constant<int, PT / 2>;
         PcbLseTile t = {}, tp = {};  // tiles of this unit and of the one before
@@ -967,6 +978,7 @@ lse_tmem_persistent_kernel(const float* __restrict__ src, const float* __restric
                     wait_rows(q + 1);
                     load(q + 1, last ? ((u + 1) % num_slices) * NS : b0, last ? tiles[(u + 1) / num_slices].k_cnt : t.k_cnt, Z{});
                 }
+                if (MODE != 0 && last) prefetch_aux(t, b0);
                 // D's slot: what chunk q - 2 left there
                 if (i == 0) {
                     if (u > u0) finish(q - 1, tp, nchp, b0p);

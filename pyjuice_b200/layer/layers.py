@@ -269,9 +269,9 @@ def _tc05_long(src, src2, aux, out, ld, B, pack, table, ranges, krow, mode, prec
     # One launch of the tensor-memory form, persistent where every SM has a (tile, 128-sample
     # slice), or by 128-term chunks; the autotuner decides, the first is the static default.
     # Measured (us, forward, weights packed, graph-timed, chunks / cluster / persistent): 200
-    # regions of 256 x 256, batch 512: 370 / 148 / 88, batch 32: 29.7 / 34.8 / 24.2; one of 2048
-    # x 2048, batch 512: 106 / 77 / 57, batch 64: 17.9 / 28.9 / 53.7; one of 512 x 512, batch 512:
-    # 11.8 / 9.6 / 16.3.
+    # regions of 256 x 256, batch 512: 315 / 135 / 88, batch 32: 29.8 / 34.0 / 24.3; one of 2048
+    # x 2048, batch 512: 105 / 72 / 57, batch 64: 17.5 / 28.3 / 53.5; one of 512 x 512, batch 512:
+    # 11.9 / 9.1 / 16.3.
     ks = _tmem_ksplit(tiles.size(0), tile_rows, index.size(1), B)
     cands = [("tm", ks), ("tm", 0), ("chunks", 0)]
     if tiles.size(0) * -(-B // 128) >= _num_sms():
@@ -344,15 +344,14 @@ def _tc05_call(src, src2, aux, out, ld, B, pack, tiles, krow, mode, prec, stream
         # static default: the persistent kernel once the layer has a unit per SM
         cands = ws_c + cands if nt * -(-B // ws_bt) >= _num_sms() else cands + ws_c
     if prec != 3 and SumLayer.tmem is None:
-        # the tensor-memory form (two CTAs per SM), the default once a 128-sample slice of every
-        # third tile runs per SM; persistent only where every SM has a unit. Measured (us,
-        # forward, graph-timed, best other / two CTAs / persistent): 119 tiles of 128 x 128,
-        # batch 512: 35.8 / 19.2 / 20.5, batch 200: 18.2 / 9.8 / 12.3; 25 tiles, batch 512: 11.3 /
-        # 7.9 / 7.5; 12 tiles: 7.5 / 7.6 / 7.0; 6 tiles: 5.4 / 7.1 / 7.0.
-        units = nt * -(-B // 128)
-        cands = [("tm", 1)] + cands if 3 * units >= _num_sms() else cands + [("tm", 1)]
-        if units >= _num_sms():
-            cands.append(("tm", 0))
+        # the tensor-memory forms, the default (two CTAs per SM) once every third SM has a (tile,
+        # 128-sample slice). Measured (us, forward, graph-timed, best other / two CTAs /
+        # persistent): 119 tiles of 128 x 128, batch 512: 35.9 / 18.1 / 20.2, batch 200: 18.4 / 9.7 /
+        # 12.2; 25 tiles, batch 512: 11.4 / 7.5 / 7.5; 12 tiles: 7.5 / 7.3 / 6.8; 6 tiles: 6.9 /
+        # 6.7 / 6.8. Persistent is offered below a unit per SM too: element flows of 25 tiles take
+        # 13.8 / 10.3 / 8.4.
+        tm = [("tm", 1), ("tm", 0)]
+        cands = tm + cands if 3 * nt * -(-B // 128) >= _num_sms() else cands + tm
     run(TUNER.pick(("tc05", mode, prec, nt, B), cands, run))
 
 
@@ -556,7 +555,7 @@ class SumLayer(Layer):
     tmem = None
     # node flows x samples from which a backward that may not modify the flows writes log f -
     # log m to a workspace first (measured, us with / without: 200 regions of 256 x 256, batch 512:
-    # 468 / 610; 119 of 128 x 128: 104 / 109; 25 of 128 x 128: 97 / 82, bound by the host)
+    # 297 / 447; 119 of 128 x 128: 87 / 95; 25 of 128 x 128: 50 / 37, bound by the host)
     ratio_min_values = 1 << 22
     tc05_long = True      # tiles of more than 128 terms as accumulating tcgen05 chunks (BF16 / E4M3 forms)
     chunk_partials = True  # all chunks of a layer in one launch into partial rows, then pcb_chunk_combine
