@@ -105,6 +105,16 @@ int pcb_status_selftest(int32_t spin_limit, void* stream);
 int pcb_fill_rows(float* mat, int64_t ld, int64_t row0, int64_t row1, float value, void* stream);
 
 /*
+ * Root flows of a gradient of the log-likelihoods: with S = sum of grad[r * s_r + b * s_b]
+ * over r < R, b < B (R * B <= 2^30), node_flows[r * ld + b] = w = grad / S * B (log w if
+ * logspace_flows != 0) and, if cum is given, *cum += sum of w. The sums are FP64. Replaces the
+ * normalisation in the gradient hook and the root rows' initialisation
+ * (src/pyjuice/model/tensorcircuit.py:24-37).
+ */
+int pcb_root_flows(const float* grad, int64_t s_r, int64_t s_b, int32_t R, int32_t B, float* node_flows, int64_t ld,
+                   int32_t logspace_flows, double* cum, void* stream);
+
+/*
  * Categorical input layer forward: node_mars[node_offset + n, b] =
  *   log(params[s_pids[n] + data[vids[n] * data_ld + b]]) for n < num_nodes, b < B
  * (NaN where the category is outside [0, ncats[n]), reported as PCB_STATUS_BAD_CATEGORY),

@@ -91,6 +91,8 @@ _SIGS = {
     "pcb_device_status": ([c_void_p, c_int32, c_void_p], c_int32),
     "pcb_status_selftest": ([c_int32, c_void_p], c_int32),
     "pcb_fill_rows": ([c_void_p, c_int64, c_int64, c_int64, c_float, c_void_p], c_int32),
+    "pcb_root_flows": ([c_void_p, c_int64, c_int64, c_int32, c_int32, c_void_p, c_int64, c_int32, c_void_p,
+                        c_void_p], c_int32),
     "pcb_input_cat_fwd": ([c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_void_p, c_int32, c_int32, c_void_p,
                            c_int64, c_int32, c_void_p, c_int64, c_int64, c_void_p], c_int32),
     "pcb_input_cat_bwd": ([c_void_p, c_int64, c_void_p, c_int64, c_int32, c_void_p, c_void_p, c_void_p, c_void_p,

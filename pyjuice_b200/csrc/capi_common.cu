@@ -92,6 +92,60 @@ __global__ void ll_sum_kernel(const float* __restrict__ lls, int B, double* __re
     }
 }
 
+// Root flows of a gradient of the log-likelihoods, g [R, B] (strides s_r, s_b): with S the sum
+// of g, nf[r, b] = w = g / S * B (its logarithm if LOG), and *cum (if given) += the sum of w.
+// Both sums are FP64 in a fixed order.
+//
+// Bound by latency: a few hundred values, for which seven element-wise and reduction launches
+// took their launch time (64 values: 1.9 us, against 10.6 us on the device and 64 us with the
+// host's share). One CTA, which holds up to kRootKeep values per thread between the
+// two sums.
+constexpr int kRootThreads = 1024;
+constexpr int kRootKeep = 8;
+
+__device__ double root_block_sum(double v, double* part) {
+    v = pcb::warp_sum(v);
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = v;
+    __syncthreads();
+    return pcb::warp_sum((threadIdx.x & 31) < (blockDim.x >> 5) ? part[threadIdx.x & 31] : 0.0);
+}
+
+template <bool LOG>
+__global__ void __launch_bounds__(kRootThreads)
+root_flows_kernel(const float* __restrict__ g, int64_t s_r, int64_t s_b, int R, int B, float* __restrict__ nf,
+                  int64_t ld, double* __restrict__ cum) {
+    pcb::pdl_begin();
+    __shared__ double part[32];
+    const int n = R * B;
+    float keep[kRootKeep];
+    double s = 0.0;
+#pragma unroll
+    for (int j = 0; j < kRootKeep; ++j) {
+        const int i = threadIdx.x + j * blockDim.x;
+        keep[j] = i < n ? g[i / B * s_r + i % B * s_b] : 0.f;
+        s += (double)keep[j];
+    }
+    for (int i = threadIdx.x + kRootKeep * blockDim.x; i < n; i += blockDim.x) s += (double)g[i / B * s_r + i % B * s_b];
+    const float total = (float)root_block_sum(s, part);
+    double c = 0.0;
+    auto emit = [&](int i, float x) {
+        const float w = x / total * (float)B;
+        nf[i / B * ld + i % B] = LOG ? logf(w) : w;
+        c += (double)w;
+    };
+#pragma unroll
+    for (int j = 0; j < kRootKeep; ++j) {
+        const int i = threadIdx.x + j * blockDim.x;
+        if (i < n) emit(i, keep[j]);
+    }
+    for (int i = threadIdx.x + kRootKeep * blockDim.x; i < n; i += blockDim.x) emit(i, g[i / B * s_r + i % B * s_b]);
+    if (cum) {
+        c = root_block_sum(c, part);
+        if (threadIdx.x == 0) *cum += c;
+    }
+}
+
 // One CTA waits, with a bounded number of polls, on an mbarrier that nothing completes (the
 // same bounded wait the tcgen05 contraction uses for its weight copy and MMAs), then reports
 // the timeout in the status word and returns.
@@ -151,6 +205,18 @@ int pcb_fill_rows(float* mat, int64_t ld, int64_t row0, int64_t row1, float valu
     return pcb::launch_status(pcb::launch_k(fill_rows_kernel, dim3((unsigned)blocks), dim3(256), 0,
                                             pcb::as_stream(stream), 1u, mat + row0 * ld, n, value),
                               "pcb_fill_rows");
+}
+
+int pcb_root_flows(const float* grad, int64_t s_r, int64_t s_b, int32_t R, int32_t B, float* node_flows, int64_t ld,
+                   int32_t logspace_flows, double* cum, void* stream) {
+    if (!grad || !node_flows || R <= 0 || B <= 0 || ld < B || s_r < 0 || s_b < 0 || (int64_t)R * B > (1 << 30))
+        return pcb::set_error(PCB_E_ARG, "pcb_root_flows: bad arguments");
+    const int64_t warps = pcb::cdiv((int64_t)R * B, 32);
+    const unsigned threads = warps < kRootThreads / 32 ? 32u * (unsigned)warps : kRootThreads;
+    return pcb::launch_status(pcb::launch_k(logspace_flows ? root_flows_kernel<true> : root_flows_kernel<false>,
+                                            dim3(1), dim3(threads), 0, pcb::as_stream(stream), 1u, grad, s_r, s_b, R,
+                                            B, node_flows, ld, cum),
+                              "pcb_root_flows");
 }
 
 int pcb_ll_sum_f64(const float* lls, int64_t ld, int32_t B, int64_t row, double* out, void* stream) {
