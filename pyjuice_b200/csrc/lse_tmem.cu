@@ -29,8 +29,8 @@
 // (70 MB): 18.1 us, 3.9 TB/s, against 35.9 us for the best of the forms that keep the samples in
 // shared memory (lse_tc05.cu); 200 regions of 256 x 256 (262 MB): 87.8 us, 3.0 TB/s, on the
 // persistent form below, against 315 us in 128-term chunks; element flows of the same layer
-// (367 MB): 113 us (139 us without the element values' prefetch), against
-// 452 us. What is left: a chunk costs about
+// (367 MB): 105 us (139 us without the element values' prefetch and with the next rows'
+// loads after the conversion), against 448 us. What is left: a chunk costs about
 // 2,000 cycles of MMAs (three products), as many of exponentials, and its rows arrive at about
 // 20 bytes per SM and cycle.
 //
@@ -944,21 +944,41 @@ lse_tmem_persistent_kernel(const float* __restrict__ src, const float* __restric
                 for (int j = 1; j < PT; ++j) m = fmaxf(m, v[j]);
                 float* pm = sPart + (q & 1) * 4 * NS + s;
                 pm[part * NS] = m;
-                asm volatile("bar.sync 1, 512;\n" ::: "memory");
-                m = fmaxf(fmaxf(fmaxf(pm[0], pm[NS]), fmaxf(pm[2 * NS], pm[3 * NS])), mrun);
-                mrun = m;
                 // A's slot: the MMAs of chunk q - AS have read it
                 if (q >= AS && !mbar_wait_bounded(barM + ((q - AS) & 1), (uint32_t)(((q - AS) >> 1) & 1))) fail = true;
                 fence_after_sync();
-                const float mu = m == -INFINITY ? 0.f : m;
-                const uint64_t nmu = pair(-mu, -mu);
+                // The values wait for the maximum in the columns that their first two parts will
+                // take, and the next chunk's rows are on their way while they are converted.
                 const uint32_t ta = a_cols(q) + tlane + part * (PT / 2);
 #pragma unroll
                 for (int g = 0; g < PT; g += 16) {
+                    uint32_t raw[2][8];
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) raw[j / 8][j % 8] = __float_as_uint(v[g + j]);
+                    tmem_st8(ta + g / 2, raw[0]);
+                    tmem_st8(ta + kColsA + g / 2, raw[1]);
+                }
+                const bool last = i + 1 == nch;
+                if (!last || u + 1 < u1) {
+                    wait_rows(q + 1);
+                    load(q + 1, last ? ((u + 1) % num_slices) * NS : b0, last ? tiles[(u + 1) / num_slices].k_cnt : t.k_cnt, Z{});
+                }
+                wait_st();
+                asm volatile("bar.sync 1, 512;\n" ::: "memory");
+                m = fmaxf(fmaxf(fmaxf(pm[0], pm[NS]), fmaxf(pm[2 * NS], pm[3 * NS])), mrun);
+                mrun = m;
+                const float mu = m == -INFINITY ? 0.f : m;
+                const uint64_t nmu = pair(-mu, -mu);
+#pragma unroll
+                for (int g = 0; g < PT; g += 16) {
+                    float raw[2][8];
+                    tmem_ld8(ta + g / 2, raw[0]);
+                    tmem_ld8(ta + kColsA + g / 2, raw[1]);
+                    wait_ld();
                     uint32_t parts[NP][8];
 #pragma unroll
                     for (int j = 0; j < 8; ++j) {
-                        const uint64_t x = mul2(add2(pair(v[g + 2 * j], v[g + 2 * j + 1]), nmu), log2e);
+                        const uint64_t x = mul2(add2(pair(raw[j / 4][2 * j % 8], raw[j / 4][2 * j % 8 + 1]), nmu), log2e);
                         const float2 x2 = unpair(x);
                         uint64_t e = pair(ex2(x2.x), ex2(x2.y));
 #pragma unroll
@@ -971,12 +991,6 @@ lse_tmem_persistent_kernel(const float* __restrict__ src, const float* __restric
                     }
 #pragma unroll
                     for (int p = 0; p < NP; ++p) tmem_st8(ta + p * kColsA + g / 2, parts[p]);
-                }
-                // the next chunk's rows
-                const bool last = i + 1 == nch;
-                if (!last || u + 1 < u1) {
-                    wait_rows(q + 1);
-                    load(q + 1, last ? ((u + 1) % num_slices) * NS : b0, last ? tiles[(u + 1) / num_slices].k_cnt : t.k_cnt, Z{});
                 }
                 if (MODE != 0 && last) prefetch_aux(t, b0);
                 // D's slot: what chunk q - 2 left there
