@@ -26,13 +26,13 @@
 // that 16 chunks accumulated in D would be 1.3e-5 too small, against 3e-7 this way.
 //
 // Measured (forward, split form, weights packed, graph-timed): 119 tiles of 128 x 128, batch 512
-// (70 MB): 18.1 us, 3.9 TB/s, against 35.9 us for the best of the forms that keep the samples in
-// shared memory (lse_tc05.cu); 200 regions of 256 x 256 (262 MB): 87.8 us, 3.0 TB/s, on the
-// persistent form below, against 315 us in 128-term chunks; element flows of the same layer
-// (367 MB): 105 us (139 us without the element values' prefetch and with the next rows'
-// loads after the conversion), against 448 us. What is left: a chunk costs about
-// 2,000 cycles of MMAs (three products), as many of exponentials, and its rows arrive at about
-// 20 bytes per SM and cycle.
+// (70 MB): 18.3 us, 3.8 TB/s, against 33.9 us for the best of the forms that keep the samples in
+// shared memory (lse_tc05.cu); 200 regions of 256 x 256 (262 MB): 83.4 us, 3.1 TB/s, on the
+// persistent form below, against 305 us in 128-term chunks; element flows of the same layer
+// (367 MB): 105.6 us (139 us without the element values' prefetch and with the next rows'
+// loads after the conversion), against 444 us. What is left of a chunk there, about 6,000 cycles:
+// 1,800 until its rows are requested (a SM takes about 37 bytes per cycle), 1,200 of
+// exponentials, up to 1,500 of sums or results, 900 of maxima and waits.
 //
 // Every wait is bounded; a CTA whose wait runs out writes NaN rows and reports
 // PCB_STATUS_WAIT_TIMEOUT.
@@ -623,31 +623,42 @@ lse_tmem_kernel(const float* __restrict__ src, const float* __restrict__ src2, c
 // in shared memory (for the same reason as above). Consecutive slices of a tile reuse its
 // weights.
 //
+// A SM takes a 128-byte load of 32 lanes every 4.5 cycles: 2,300 of a chunk's cycles. Values
+// (mode 0) therefore come as 16-byte asynchronous copies through shared memory (COPY), one
+// instruction per row: 200 regions of 256 x 256 86.8 -> 83.4 us, 1 of 2048 x 2048 57.5 -> 51.8, FP32
+// 119 of 128 x 128 with the pack 46.8 -> 41.6. Element flows keep the loads (copied: 119 tiles 32.4
+// against 31.2, 200 regions 105.0 against 105.2): their registers spill. Bulk copies of a row (512
+// bytes) take 100 cycles each (156 us); three loader warps have too few copies in flight (88 us).
+//
 // NP parts per operand: 1 single bf16, 2 split (hi, lo), 3 for the plain FP32 form (hi, mid, lo:
 // 24 bits; the six products down to 2^-18, smallest first, then hi * hi alone truncates). With
 // three parts A has one slot, D's two hold one chunk, whose sums go to shared memory when another
 // follows, and the weights then have one slot too. 119 tiles of 128 x
-// 128, batch 512, FP32: 47 us with the pack against 102 us for FFMA; error against FP64 no larger (element flows 3.04e-7
-// against 3.06e-7).
+// 128, batch 512, FP32: 40 us with the pack against 102 us for FFMA; error against FP64 no larger
+// (element flows 3.04e-7 against 3.06e-7).
 constexpr int kPWarps = 16;
 constexpr int kPThreads = 32 * kPWarps + 32;
 constexpr int PT = KT / 4;  // terms per thread and chunk
 constexpr int EB = 8;       // accumulator columns per epilogue step
 constexpr int kRowRing = 4;
+constexpr uint32_t kPSlots = 216 * 1024;  // shared memory for weights, sums and values
 
 struct PSmem {
-    uint32_t wslot, sum, part, rows, bar, slot, total;  // the weight slots come first
+    uint32_t wslot, sum, vals, part, rows, bar, slot, total;  // the weight slots come first
     int nw;
-    __host__ __device__ PSmem(int n_pad, int np, bool sums) {
+    __host__ __device__ PSmem(int n_pad, int np, bool sums, bool copied) {
         wslot = (uint32_t)n_pad * KT * 2 * (np < 2 ? 2 : np);
-        nw = np == 3 && sums ? 1 : 2;
+        const uint32_t rest = (sums ? (uint32_t)n_pad * NS * 4 : 0) + (copied ? KT * NS * 4 : 0);
+        nw = (np == 3 && sums) || 2 * wslot + rest > kPSlots ? 1 : 2;
         sum = nw * wslot;
-        part = sum + (sums ? (uint32_t)n_pad * NS * 4 : 0);  // [2 buffers][4 parts][NS] chunk maxima
+        vals = sum + (sums ? (uint32_t)n_pad * NS * 4 : 0);  // [KT][NS] values of a chunk (copied rows)
+        part = vals + (copied ? KT * NS * 4 : 0);              // [2 buffers][4 parts][NS] chunk maxima
         rows = part + 2 * 4 * NS * 4;       // [kRowRing][KT]
         bar = rows + kRowRing * KT * 4;
         slot = bar + 16 * 8;
         total = slot + 16;
     }
+    __host__ __device__ bool fits() const { return part <= kPSlots; }
 };
 
 __device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&v)[8]) {
@@ -662,7 +673,7 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&v)[8]) {
 // exp(m - to) for a scale between maxima; equal ones (also both -inf) give 1
 __device__ __forceinline__ float rescale(float m, float to) { return m == to ? 1.f : pcb::fast_exp(m - to); }
 
-template <int MODE, int NP>
+template <int MODE, int NP, bool COPY>
 __global__ void __launch_bounds__(kPThreads, 1)
 lse_tmem_persistent_kernel(const float* __restrict__ src, const float* __restrict__ src2,
                            const float* __restrict__ aux, float* __restrict__ out, int64_t ld, int B,
@@ -673,14 +684,16 @@ lse_tmem_persistent_kernel(const float* __restrict__ src, const float* __restric
     extern __shared__ __align__(1024) uint8_t sm[];
     constexpr int AS = NP == 3 ? 1 : 2;  // slots of A
     static_assert(NP < 3 || MODE < 2, "the FP32 form takes rewritten flows");
-    const PSmem S(n_max, NP, sums);
+    const PSmem S(n_max, NP, sums, COPY);
     float* sSum = reinterpret_cast<float*>(sm + S.sum);  // [rows][samples]
+    float* sVals = reinterpret_cast<float*>(sm + S.vals);
     float* sPart = reinterpret_cast<float*>(sm + S.part);
     int* sRows = reinterpret_cast<int*>(sm + S.rows);
     uint64_t* barW = reinterpret_cast<uint64_t*>(sm + S.bar);  // [2] weights arrived
     uint64_t* barM = barW + 2;                                 // [2] MMAs completed
     uint64_t* barA = barW + 4;                                 // [2] A written, D read
     uint64_t* barR = barW + 6;                                 // [kRowRing] row numbers written
+    uint64_t* barV = barW + 10;                                // values of a chunk arrived
     uint32_t* slot = reinterpret_cast<uint32_t*>(sm + S.slot);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int u0 = (int)((int64_t)num_units * blockIdx.x / gridDim.x);
@@ -697,6 +710,7 @@ lse_tmem_persistent_kernel(const float* __restrict__ src, const float* __restric
             mbar_init(barA + i, kPWarps);
         }
         for (int i = 0; i < kRowRing; ++i) mbar_init(barR + i, 1);
+        mbar_init(barV, 32 * kPWarps);
         slot[1] = 0;
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
@@ -814,6 +828,18 @@ lse_tmem_persistent_kernel(const float* __restrict__ src, const float* __restric
         auto wait_rows = [&](int q) {
             if (!mbar_wait_bounded(barR + q % kRowRing, (uint32_t)((q / kRowRing) & 1))) fail = true;
         };
+        // COPY: this warp's eight rows of chunk q to shared memory, 16 bytes per lane; barV follows
+        auto copy = [&](int q, int b0, int nk) {
+            constexpr int n = KT / kPWarps;
+            const int* rows = sRows + (q % kRowRing) * KT + warp * n;
+            float* to = sVals + warp * n * NS + 4 * lane;
+            if (b0 + 4 * lane < B) {  // ld is a multiple of 4
+#pragma unroll
+                for (int j = 0; j < n; ++j)
+                    if (warp * n + j < nk) pcb::cp_async16(to + j * NS, src + (int64_t)rows[j] * ld + b0 + 4 * lane);
+            }
+            asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];\n" ::"r"(smem_u32(barV)) : "memory");
+        };
         // log f - log m of the terms loaded last (mode 2)
         auto to_log = [&](auto first) {
             constexpr int j0 = decltype(first)::value;
@@ -919,7 +945,12 @@ lse_tmem_persistent_kernel(const float* __restrict__ src, const float* __restric
         int q = 0, nchp = 0, b0p = 0;
         if (u0 < u1) {
             wait_rows(0);
-            load(0, (u0 % num_slices) * NS, tiles[u0 / num_slices].k_cnt, Z{});
+            const int b0 = (u0 % num_slices) * NS, nk = tiles[u0 / num_slices].k_cnt;
+            if constexpr (COPY) {
+                copy(0, b0, nk);
+            } else {
+                load(0, b0, nk, Z{});
+            }
         }
         for (int u = u0; u < u1; ++u) {
             t = tiles[u / num_slices];
@@ -928,6 +959,12 @@ lse_tmem_persistent_kernel(const float* __restrict__ src, const float* __restric
             const bool active = b0 + (warp & 3) * 32 < B;
             float mrun = -INFINITY;
             for (int i = 0; i < nch; ++i, ++q) {
+                if constexpr (COPY) {
+                    if (!mbar_wait_bounded(barV, (uint32_t)(q & 1))) fail = true;
+                    const float* p = sVals + part * PT * NS + s;
+#pragma unroll
+                    for (int j = 0; j < PT; ++j) v[j] = p[j * NS];
+                }
                 if (MODE == 2) {
                     to_log(Z{});
                     load(q, b0, t.k_cnt, H{});
@@ -947,24 +984,31 @@ lse_tmem_persistent_kernel(const float* __restrict__ src, const float* __restric
                 // A's slot: the MMAs of chunk q - AS have read it
                 if (q >= AS && !mbar_wait_bounded(barM + ((q - AS) & 1), (uint32_t)(((q - AS) >> 1) & 1))) fail = true;
                 fence_after_sync();
-                // The values wait for the maximum in the columns that their first two parts will
-                // take, and the next chunk's rows are on their way while they are converted.
                 const uint32_t ta = a_cols(q) + tlane + part * (PT / 2);
-#pragma unroll
-                for (int g = 0; g < PT; g += 16) {
-                    uint32_t raw[2][8];
-#pragma unroll
-                    for (int j = 0; j < 16; ++j) raw[j / 8][j % 8] = __float_as_uint(v[g + j]);
-                    tmem_st8(ta + g / 2, raw[0]);
-                    tmem_st8(ta + kColsA + g / 2, raw[1]);
-                }
                 const bool last = i + 1 == nch;
-                if (!last || u + 1 < u1) {
-                    wait_rows(q + 1);
-                    load(q + 1, last ? ((u + 1) % num_slices) * NS : b0, last ? tiles[(u + 1) / num_slices].k_cnt : t.k_cnt, Z{});
+                if constexpr (!COPY) {
+                    // The values wait for the maximum in the columns that their first two parts will
+                    // take, and the next chunk's rows are on their way while they are converted.
+#pragma unroll
+                    for (int g = 0; g < PT; g += 16) {
+                        uint32_t raw[2][8];
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) raw[j / 8][j % 8] = __float_as_uint(v[g + j]);
+                        tmem_st8(ta + g / 2, raw[0]);
+                        tmem_st8(ta + kColsA + g / 2, raw[1]);
+                    }
+                    if (!last || u + 1 < u1) {
+                        wait_rows(q + 1);
+                        load(q + 1, last ? ((u + 1) % num_slices) * NS : b0, last ? tiles[(u + 1) / num_slices].k_cnt : t.k_cnt, Z{});
+                    }
+                    wait_st();
                 }
-                wait_st();
                 asm volatile("bar.sync 1, 512;\n" ::: "memory");
+                if (COPY && (!last || u + 1 < u1)) {  // every warp has read chunk q's values
+                    wait_rows(q + 1);
+                    if (last) copy(q + 1, ((u + 1) % num_slices) * NS, tiles[(u + 1) / num_slices].k_cnt);
+                    else copy(q + 1, b0, t.k_cnt - (i + 1) * KT);
+                }
                 m = fmaxf(fmaxf(fmaxf(pm[0], pm[NS]), fmaxf(pm[2 * NS], pm[3 * NS])), mrun);
                 mrun = m;
                 const float mu = m == -INFINITY ? 0.f : m;
@@ -972,9 +1016,14 @@ lse_tmem_persistent_kernel(const float* __restrict__ src, const float* __restric
 #pragma unroll
                 for (int g = 0; g < PT; g += 16) {
                     float raw[2][8];
-                    tmem_ld8(ta + g / 2, raw[0]);
-                    tmem_ld8(ta + kColsA + g / 2, raw[1]);
-                    wait_ld();
+                    if constexpr (COPY) {
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) raw[j / 8][j % 8] = v[g + j];
+                    } else {
+                        tmem_ld8(ta + g / 2, raw[0]);
+                        tmem_ld8(ta + kColsA + g / 2, raw[1]);
+                        wait_ld();
+                    }
                     uint32_t parts[NP][8];
 #pragma unroll
                     for (int j = 0; j < 8; ++j) {
@@ -1038,19 +1087,27 @@ lse_tmem_persistent_kernel(const float* __restrict__ src, const float* __restric
     }
 }
 
-template <int MODE, int NP>
+template <int MODE, int NP, bool COPY>
 int launch_persistent(const float* src, const float* src2, const float* aux, float* out, int64_t ld, int B,
                       const uint8_t* packed, const PcbLseTile* tiles, int num_tiles, int n_max, const int* krow,
                       const int* chunk_index, int chunk_ld, cudaStream_t s) {
     const bool sums = chunk_index && chunk_ld > (NP == 3 ? 1 : 2);
-    const size_t smem = PSmem(n_max, NP, sums).total;
+    const PSmem S(n_max, NP, sums, COPY);
+    if constexpr (COPY) {
+        // Rows that 16-byte copies can read, a full slice of samples (below that the copies' lanes
+        // idle), and room for a chunk of values.
+        if (!pcb::vec_ok(src, ld) || B < NS || !S.fits())
+            return launch_persistent<MODE, NP, false>(src, src2, aux, out, ld, B, packed, tiles, num_tiles, n_max, krow,
+                                                      chunk_index, chunk_ld, s);
+    }
+    const size_t smem = S.total;
     static bool configured[64] = {false};
     static int sms[64] = {0};
     int dev = 0;
     cudaGetDevice(&dev);
     dev = dev < 0 ? 0 : (dev > 63 ? 63 : dev);
     if (!configured[dev]) {
-        cudaError_t e = cudaFuncSetAttribute(lse_tmem_persistent_kernel<MODE, NP>,
+        cudaError_t e = cudaFuncSetAttribute(lse_tmem_persistent_kernel<MODE, NP, COPY>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
         if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms[dev], cudaDevAttrMultiProcessorCount, dev);
         if (e != cudaSuccess) return pcb::set_error(PCB_E_CUDA, "pcb_lse_contract_tmem: %s", cudaGetErrorString(e));
@@ -1060,7 +1117,7 @@ int launch_persistent(const float* src, const float* src2, const float* aux, flo
     const int64_t units = (int64_t)num_tiles * slices;
     if (units > INT32_MAX) return pcb::set_error(PCB_E_ARG, "pcb_lse_contract_tmem: too many tiles");
     return pcb::launch_status(
-        pcb::launch_k(lse_tmem_persistent_kernel<MODE, NP>, dim3((unsigned)std::min<int64_t>(units, sms[dev])),
+        pcb::launch_k(lse_tmem_persistent_kernel<MODE, NP, COPY>, dim3((unsigned)std::min<int64_t>(units, sms[dev])),
                       dim3(kPThreads), smem, s, 1u, src, src2, aux, out, ld, B, packed, tiles, krow, chunk_index,
                       chunk_ld, n_max, sums, slices, (int)units, pcb::status_word()),
         "pcb_lse_contract_tmem");
@@ -1111,7 +1168,7 @@ extern "C" int pcb_lse_contract_tmem(const float* src, const float* src2, const 
     cudaStream_t s = pcb::as_stream(stream);
     if (ksplit == 0) {
 #define PCB_TP(M, P) \
-    launch_persistent<M, P>(src, src2, aux, out, ld, B, packed, tiles, num_tiles, n_max, krow, chunk_index, chunk_ld, s)
+    launch_persistent<M, P, M == 0>(src, src2, aux, out, ld, B, packed, tiles, num_tiles, n_max, krow, chunk_index, chunk_ld, s)
         if (prec == 0) return mode == 0 ? PCB_TP(0, 3) : PCB_TP(1, 3);
         if (prec == 1) return mode == 0 ? PCB_TP(0, 1) : (mode == 1 ? PCB_TP(1, 1) : PCB_TP(2, 1));
         return mode == 0 ? PCB_TP(0, 2) : (mode == 1 ? PCB_TP(1, 2) : PCB_TP(2, 2));

@@ -269,9 +269,9 @@ def _tc05_long(src, src2, aux, out, ld, B, pack, table, ranges, krow, mode, prec
     # One launch of the tensor-memory form, persistent where every SM has a (tile, 128-sample
     # slice), or by 128-term chunks; the autotuner decides, the first is the static default.
     # Measured (us, forward, weights packed, graph-timed, chunks / cluster / persistent): 200
-    # regions of 256 x 256, batch 512: 315 / 135 / 88, batch 32: 29.8 / 34.0 / 24.3; one of 2048
-    # x 2048, batch 512: 105 / 72 / 57, batch 64: 17.5 / 28.3 / 53.5; one of 512 x 512, batch 512:
-    # 11.9 / 9.1 / 16.3.
+    # regions of 256 x 256, batch 512: 305 / 135 / 83, batch 32: 29.7 / 34.1 / 24.6; one of 2048
+    # x 2048, batch 512: 105 / 72 / 52, batch 64: 17.5 / 28.2 / 55.4; one of 512 x 512, batch 512:
+    # 11.9 / 9.2 / 15.5.
     ks = _tmem_ksplit(tiles.size(0), tile_rows, index.size(1), B)
     cands = [("tm", ks), ("tm", 0), ("chunks", 0)]
     if tiles.size(0) * -(-B // 128) >= _num_sms():
@@ -346,10 +346,9 @@ def _tc05_call(src, src2, aux, out, ld, B, pack, tiles, krow, mode, prec, stream
     if prec != 3 and SumLayer.tmem is None:
         # the tensor-memory forms, the default (two CTAs per SM) once every third SM has a (tile,
         # 128-sample slice). Measured (us, forward, graph-timed, best other / two CTAs /
-        # persistent): 119 tiles of 128 x 128, batch 512: 35.9 / 18.1 / 20.2, batch 200: 18.4 / 9.7 /
-        # 12.2; 25 tiles, batch 512: 11.4 / 7.5 / 7.5; 12 tiles: 7.5 / 7.3 / 6.8; 6 tiles: 6.9 /
-        # 6.7 / 6.8. Persistent is offered below a unit per SM too: element flows of 25 tiles take
-        # 13.8 / 10.3 / 8.4.
+        # persistent): 119 tiles of 128 x 128, batch 512: 33.9 / 18.3 / 19.6, batch 200: 18.4 / 9.8 /
+        # 11.8; 25 tiles, batch 512: 11.4 / 7.6 / 7.3; 12 tiles: 7.6 / 7.3 / 6.6. Persistent is offered
+        # below a unit per SM too: element flows of 25 tiles take 13.8 / 10.3 / 8.7.
         tm = [("tm", 1), ("tm", 0)]
         cands = tm + cands if 3 * nt * -(-B // 128) >= _num_sms() else cands + tm
     run(TUNER.pick(("tc05", mode, prec, nt, B), cands, run))
@@ -776,8 +775,8 @@ class SumLayer(Layer):
         """Whether an FP32 contraction runs on the tensor cores in three bf16 parts (the persistent
         pcb_lse_contract_tmem): tiles of at least 64 rows and terms, and a (tile, 128-sample
         slice) for every other SM. Measured, forward with the pack against FFMA (us, batch 512):
-        200 regions of 256 x 256: 197 / 773; 119 of 128 x 128: 47 / 102; 40 of 64 x 512: 48 / 84; 25
-        of 96 x 96: 12.7 / 18.6; 100 of 32 x 32: 18.7 / 13.1."""
+        200 regions of 256 x 256: 179 / 773; 119 of 128 x 128: 40 / 102; 40 of 64 x 512: 44 / 84; 25
+        of 96 x 96: 11.6 / 18.6; 100 of 32 x 32: 18.7 / 13.1."""
         return (SumLayer.tmem is not False and SumLayer.tc05_long and tile_rows >= 64 and max_terms >= 64
                 and table is not None and tiles.size(0) >= SumLayer.tc05_min_tiles
                 and 2 * tiles.size(0) * -(-B // 128) >= _num_sms())

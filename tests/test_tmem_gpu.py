@@ -166,3 +166,39 @@ def test_lane_parameter_flows(nodes, terms, bs, B, form, children, modified, cud
     tol = (3.0 * 2.0 ** -18 if form == 2 else 2.0 ** -7) + 36 * 2.0 ** -23 + 1e-5
     assert torch.all((pf.double() - old.double() - want).abs() <= tol * want + 2.0 ** -23 * (old.double() + want))
     assert nat.device_status() == 0
+
+
+@pytest.mark.parametrize("regions,nodes,terms,bs,B", [(1, 16, 16, 16, 1), (2, 128, 128, 32, 129), (3, 80, 272, 16, 260),
+                                                      (2, 128, 656, 32, 131), (160, 32, 208, 16, 512)])
+@pytest.mark.parametrize("form", [0, 1, 2])
+def test_copied_rows(regions, nodes, terms, bs, B, form, cuda_device, settings, monkeypatch):
+    """Persistent form: rows that come as 16-byte copies (aligned rows) and rows that are loaded by
+    the threads (any other stride) go through the same arithmetic, to the bit."""
+    from pyjuice_b200.layer import layers as mod
+    SumLayer.tmem, SumLayer.tc05_min_tiles, SumLayer.ratio_min_values = 0, 1, 0
+    monkeypatch.setattr(mod, "_num_sms", lambda: 1)
+    if form:
+        SumLayer.bf16_form = form
+    layer = _layer(regions, nodes, terms, bs, cuda_device)
+    gen = torch.Generator(device=cuda_device).manual_seed(nodes + terms + B)
+    rnd = lambda *shape: torch.rand(shape, generator=gen, device=cuda_device)
+    params = torch.cat([torch.zeros([bs ** 2], device=cuda_device), rnd(regions * nodes * terms) / terms + 1e-4])
+    em = -12.0 * rnd(bs + regions * terms, B)
+    em[rnd(bs + regions * terms, B) < 0.1] = -float("inf")
+    em[:, 0] = -float("inf")
+    nf = torch.log(rnd(bs + regions * nodes, B)) + 6.0
+    got = []
+    for ld in (-(-B // 4) * 4 + 4, -(-B // 4) * 4 + 5):
+        def at(t):
+            m = torch.full([t.size(0), ld], float("nan"), device=cuda_device)  # nothing beyond B counts
+            m[:, :B] = t
+            return m[:, :B]
+        nm, ef = at(torch.full([bs + regions * nodes, B], 5.0, device=cuda_device)), at(torch.full_like(em, 9.0))
+        layer(nm, at(em), params, force_use_bf16=form != 0, force_use_fp32=form == 0)
+        layer.backward(at(nf), ef, nm, at(em), params, None, allow_modify_flows=True, _flows_modified=True,
+                       force_use_fp32=form == 0)
+        got.append((nm.clone(), ef.clone()))
+    (a, ea), (b, eb) = got
+    assert not torch.isnan(a).any() and not torch.isnan(ea).any()
+    assert torch.equal(a, b) and torch.equal(ea, eb)
+    assert nat.device_status() == 0
