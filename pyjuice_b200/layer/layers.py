@@ -351,7 +351,9 @@ def _tc05_call(src, src2, aux, out, ld, B, pack, tiles, krow, mode, prec, stream
         # below a unit per SM too: element flows of 25 tiles take 13.8 / 10.3 / 8.7.
         tm = [("tm", 1), ("tm", 0)]
         cands = tm + cands if 3 * nt * -(-B // 128) >= _num_sms() else cands + tm
-    run(TUNER.pick(("tc05", mode, prec, nt, B), cands, run))
+    # fewer forms on offer: a choice of its own (a stored one is taken whatever is on offer)
+    limited = (("workspace",) if shifted else ()) + (("no tmem",) if SumLayer.tmem is False else ())
+    run(TUNER.pick(("tc05", mode, prec, nt, B) + limited, cands, run))
 
 
 def _short_tile(key, num_tiles: int, tile_rows: int, B: int, fused: bool, run) -> None:

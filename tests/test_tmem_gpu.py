@@ -202,3 +202,32 @@ def test_copied_rows(regions, nodes, terms, bs, B, form, cuda_device, settings, 
     assert not torch.isnan(a).any() and not torch.isnan(ea).any()
     assert torch.equal(a, b) and torch.equal(ea, eb)
     assert nat.device_status() == 0
+
+
+def test_stored_choice_for_ratio_rows(cuda_device, settings, monkeypatch):
+    """A stored choice of the TMA form for a layer's rewritten flows is not taken for the ratio
+    workspace (which that form cannot read), nor one of the tensor-memory form when that is off."""
+    from pyjuice_b200.autotune import TUNER
+    SumLayer.tc05_min_tiles, SumLayer.ratio_min_values, SumLayer.tmem = 1, 0, None
+    layer = _layer(2, 128, 128, 32, cuda_device)
+    gen = torch.Generator(device=cuda_device).manual_seed(3)
+    rnd = lambda *shape: torch.rand(shape, generator=gen, device=cuda_device)
+    params = torch.cat([torch.zeros([32 ** 2], device=cuda_device), rnd(2 * 128 * 128) / 128])
+    ems, nms, nfs = -4.0 * rnd(32 + 256, 64), -rnd(32 + 256, 64), rnd(32 + 256, 64)
+
+    def flows():
+        ef = torch.zeros_like(ems)
+        layer.backward(nfs.clone(), ef, nms, ems, params, None)
+        return ef
+
+    with monkeypatch.context() as m:
+        m.setattr(TUNER, "choices", {})
+        want = flows()
+    for tmem, choice in ((None, ("ws", 64)), (False, ("tm", 9))):  # 9: no such form
+        SumLayer.tmem = tmem
+        nt = layer._desc(torch.device(cuda_device))["el_groups"][0]["tiles"].size(0)
+        with monkeypatch.context() as m:
+            m.setattr(TUNER, "choices", {"|".join(map(str, ("tc05", 1, 2, nt, 64))): choice})
+            # split operands: the forms differ by their summation order and approximations
+            assert torch.all((flows() - want).abs() <= 2e-5 * want.abs() + 1e-12)
+    assert nat.device_status() == 0
