@@ -143,6 +143,9 @@ def _pack3(holder: dict, table: torch.Tensor) -> torch.Tensor:
     return h["pack3"]
 
 
+kTmemCluster = 8  # most CTAs that share a tile in pcb_lse_contract_tmem
+
+
 def _tmem_ksplit(num_tiles: int, tile_rows: int, num_chunks: int, B: int) -> int:
     """CTAs (a cluster) that share a tile's chunks in pcb_lse_contract_tmem (``ksplit``). Tiles
     of more than 64 rows: one per chunk, so that two CTAs fit on an SM (the sums of several
@@ -150,6 +153,17 @@ def _tmem_ksplit(num_tiles: int, tile_rows: int, num_chunks: int, B: int) -> int
     if tile_rows > 64:
         return num_chunks if num_chunks < 6 else 8
     return max(1, min(8, num_chunks, 2 * _num_sms() // (num_tiles * -(-B // 128))))
+
+
+def _tmem_pays(sub_tiles: int, B: int) -> bool:
+    """Whether the tensor-memory forms are offered for a BF16 contraction of so many (128 x 128)
+    sub-tiles: from about a 32-sample slice of one per SM. Below, their 128-sample slices leave SMs
+    idle, and timings of single eager launches (which the host bounds there) do not tell the forms
+    apart. Measured (us in a graph, best other form / best of these): 119 tiles, batch 32: 5.5 /
+    7.5, batch 64: 7.7 / 7.6; 60 tiles, batch 64: 5.4 / 6.9, batch 200: 11.3 / 7.8; 12 tiles, batch
+    200: 5.2 / 7.0, batch 512: 7.6 / 6.6. 16 forward steps of an HMM of 384 states, batch 200: 186 /
+    203, 512: 221 / 206; of 512 states, batch 256: 190 / 193, 512: 274 / 234."""
+    return 8 * sub_tiles * -(-B // 32) >= 7 * _num_sms()
 
 
 class _ShiftedRows:
@@ -266,6 +280,17 @@ def _tc05_long(src, src2, aux, out, ld, B, pack, table, ranges, krow, mode, prec
         return chunks()
     if SumLayer.tmem is not None:
         return tmem(SumLayer.tmem)
+    sub_tiles = tiles.size(0) * index.size(1)
+    if sub_tiles < SumLayer.tc05_min_tiles:
+        # One launch; chunks and their combination take two. Measured (us, one region, batch 200,
+        # eager forward with the pack, mma.sync / chunks / this): 160 x 160: 21.8 / 33.9 / 18.8, 256 x
+        # 256: 32.7 / 31.8 / 18.6; 16 forward steps of an HMM in a graph: 160 states 370 / 163 / 187,
+        # 256 states 533 / 168 / 194.
+        return tmem(_tmem_ksplit(tiles.size(0), tile_rows, index.size(1), B))
+    # up to 128 samples, chunks in parallel beat eight CTAs with several chunks each (one of 2048 x
+    # 2048, batch 64, below)
+    if not _tmem_pays(sub_tiles, B) or (index.size(1) > kTmemCluster and B <= 128):
+        return chunks()
     # One launch of the tensor-memory form, persistent where every SM has a (tile, 128-sample
     # slice), or by 128-term chunks; the autotuner decides, the first is the static default.
     # Measured (us, forward, weights packed, graph-timed, chunks / cluster / persistent): 200
@@ -343,7 +368,7 @@ def _tc05_call(src, src2, aux, out, ld, B, pack, tiles, krow, mode, prec, stream
         ws_c = [("ws", ws_bt), ("ws", 96 - ws_bt)]
         # static default: the persistent kernel once the layer has a unit per SM
         cands = ws_c + cands if nt * -(-B // ws_bt) >= _num_sms() else cands + ws_c
-    if prec != 3 and SumLayer.tmem is None:
+    if prec != 3 and SumLayer.tmem is None and _tmem_pays(nt, B):
         # the tensor-memory forms, the default (two CTAs per SM) once every third SM has a (tile,
         # 128-sample slice). Measured (us, forward, graph-timed, best other / two CTAs /
         # persistent): 119 tiles of 128 x 128, batch 512: 33.9 / 18.3 / 19.6, batch 200: 18.4 / 9.8 /
@@ -766,11 +791,18 @@ class SumLayer(Layer):
     def _fw_long(self, d, prec):
         """Whether the forward runs its tiles of more than 128 terms as tcgen05 chunks."""
         return (prec > 0 and SumLayer.tc05_long and not d["fw_short"] and d["fw_ch"] is not None
-                and d["fw_ch"].size(0) >= SumLayer.tc05_min_tiles)
+                and self._enough_chunks(d["fw_ch"], prec))
 
     def _el_long(self, eg, prec):
         return (prec > 0 and SumLayer.tc05_long and not eg["short"] and eg["ch"] is not None
-                and eg["ch"].size(0) >= SumLayer.tc05_min_tiles)
+                and self._enough_chunks(eg["ch"], prec))
+
+    @staticmethod
+    def _enough_chunks(ch, prec):
+        """Long tiles run on tcgen05 from two 128-term chunks on (at the default tc05_min_tiles): the
+        chunks run side by side where the mma.sync kernel walks them (figures at _tc05_long). E4M3, which rounds more than
+        that kernel, from tc05_min_tiles."""
+        return (1 if prec == 3 else 3) * ch.size(0) >= SumLayer.tc05_min_tiles
 
     @staticmethod
     def _f32_tmem(tiles, tile_rows, max_terms, table, B):

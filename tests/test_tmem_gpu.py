@@ -231,3 +231,35 @@ def test_stored_choice_for_ratio_rows(cuda_device, settings, monkeypatch):
             # split operands: the forms differ by their summation order and approximations
             assert torch.all((flows() - want).abs() <= 2e-5 * want.abs() + 1e-12)
     assert nat.device_status() == 0
+
+
+@pytest.mark.parametrize("nodes,terms,bs,B", [(16, 144, 16, 16), (160, 160, 32, 33), (256, 256, 32, 64), (64, 320, 64, 512)])
+def test_few_long_tiles(nodes, terms, bs, B, cuda_device):
+    """One region of two to five 128-term chunks, default settings: split operands as in
+    test_contractions, on whichever form the rules take."""
+    layer = _layer(1, nodes, terms, bs, cuda_device)
+    d = layer._desc(torch.device(cuda_device))
+    assert layer._fw_long(d, 2) and layer._fw_long(d, 3) == (d["fw_ch"].size(0) >= 6)
+    gen = torch.Generator(device=cuda_device).manual_seed(nodes + B)
+    rnd = lambda *shape: torch.rand(shape, generator=gen, device=cuda_device)
+    w = torch.exp(-4.0 * rnd(nodes, terms))
+    w = w / w.sum(dim=1, keepdim=True)
+    params = torch.cat([torch.zeros([bs ** 2], device=cuda_device),
+                        w.reshape(nodes // bs, bs, terms).permute(0, 2, 1).reshape(-1)])
+    em = -12.0 * rnd(terms, B)
+    em[:, 0] = -float("inf")
+    ems = torch.cat([torch.full([bs, B], -float("inf"), device=cuda_device), em])
+    nm = torch.zeros([bs + nodes, B], device=cuda_device)
+    layer(nm, ems, params, force_use_bf16=True)
+    ref = torch.log(w.double() @ em.double().exp())
+    got = nm[bs:].double()
+    assert torch.equal(torch.isinf(got), torch.isinf(ref))
+    fin = torch.isfinite(ref)
+    assert torch.all((got - ref)[fin].abs() <= 2e-5 + 4e-7 * ref[fin].abs())
+    nms = torch.cat([torch.zeros([bs, B], device=cuda_device), ref.float()])
+    nf = torch.softmax(3.0 * rnd(nodes, B), dim=0)
+    ef = torch.zeros_like(ems)
+    layer.backward(torch.cat([torch.zeros([bs, B], device=cuda_device), nf]), ef, nms, ems, params, None)
+    ratio = torch.where(fin, nf.double() * torch.exp(-ref), 0.0)
+    want = (w.double().T @ ratio) * em.double().exp()
+    assert torch.all((ef[bs:].double() - want).abs() <= 3e-5 * want)
