@@ -53,8 +53,8 @@ BATCH = 512
 STEP_SIZE = 0.1
 PSEUDOCOUNT = 0.1
 # DRAM bytes (read + written) of the roofline launch, the largest layer's parameter flows,
-# from one ncu capture of `bench.py --profile-step` (-k regex:sum_pflows -s 63 -c 1).
-PFLOW_TRAFFIC_BYTES = 81_879_552
+# from one ncu capture of `bench.py --profile-step` (-k regex:sum_pflows_lanes, 238 CTAs).
+PFLOW_TRAFFIC_BYTES = 78_281_984
 METRIC = "EM samples/s (fwd+bwd+update) 1xB200, BF16-TC vs FP32 plain; dLL vs FP64 oracle"
 WORKLOAD = "HCLT 28x28 vars x 256 cats, 128 latents, block 32, EM step (fwd+bwd+mini_batch_em)"
 
@@ -888,12 +888,12 @@ def main():
         step(data_dev[:B], {"force_use_bf16": True})  # node flows of the full batch (rewritten as log f - log m)
         pf = pflows_roofline(pc)
         achieved = pf["bytes"] / pf["seconds"] / 1e9
-        roof = {"kernel": "pcb_sum_pflows (sum_pflows_kernel, split-bf16 form, 64-child tiles) of the largest "
+        roof = {"kernel": "pcb_sum_pflows_lanes (autotuned, split-bf16 form, 64-child tiles) of the largest "
                           "sum layer: the kernel with the largest share of the step",
                 "bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s", "frac": achieved / hbm,
                 "traffic": PFLOW_TRAFFIC_BYTES,
                 "traffic_source": "dram__bytes_read.sum + dram__bytes_write.sum of this launch, one ncu capture "
-                                  "of bench.py --profile-step (-k regex:sum_pflows -s 63 -c 1)",
+                                  "of bench.py --profile-step (-k regex:sum_pflows_lanes, 238 CTAs)",
                 "peak_source": f"{src} hbm_gbs (of measured)" if src == "measured" else f"{src} hbm_gbs",
                 "alg_bytes_per_launch": pf["bytes"], "us_per_launch": pf["seconds"] * 1e6,
                 "tensor_tflops_achieved": pf["flops"] / pf["seconds"] / 1e12,

@@ -842,8 +842,8 @@ lse_tmem_persistent_kernel(const float* __restrict__ src, const float* __restric
         };
         // log f - log m of the terms loaded last (mode 2)
         auto to_log = [&](auto first) {
-            constexpr int j0 = decltype(first)::value;
             if constexpr (MODE == 2) {
+                constexpr int j0 = decltype(first)::value;
                 float f[NL];
 #pragma unroll
                 for (int j = 0; j < NL; ++j) f[j] = v[j0 + j];
