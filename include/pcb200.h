@@ -376,7 +376,7 @@ int pcb_pack_weights(const float* params, const PcbLseTile* tiles, int32_t num_t
 
 /*
  * The weights of the same tiles in three bf16 parts (hi, mid, lo: 24 bits), 98304 bytes per
- * tile: the operand of pcb_lse_contract_tmem's FP32 form.
+ * tile: the operand of pcb_lse_contract_tmem's three-part form.
  */
 int pcb_pack_weights_f32(const float* params, const PcbLseTile* tiles, int32_t num_tiles, int32_t rows_per_block,
                          const int32_t* kw, int32_t w_stride, uint8_t* packed, void* stream);
@@ -453,8 +453,9 @@ int pcb_lse_contract_tc05_accum(const float* src, const float* src2, const float
 /*
  * pcb_lse_contract for tiles of any number of terms, in one launch, with the samples along the
  * tensor-memory lanes: the BF16 forms (prec 1: single operands, 2: split), and, persistent
- * (ksplit 0) for modes 0 and 1, the plain FP32 form (prec 0, operands in three parts packed by
- * pcb_pack_weights_f32, 98304 bytes per tile). `packed`
+ * (ksplit 0) for modes 0 and 1, a form with operands in three bf16 parts (prec 0, packed by
+ * pcb_pack_weights_f32, 98304 bytes per tile; truncated sums, and fewer bits for terms more
+ * than 75 nats below their tile's largest). `packed`
  * holds the tiles' weights (pcb_pack_weights): of tile t itself (chunk_index NULL, tiles of
  * at most 128 terms), or of its 128-term chunk j at packed + chunk_index[t * chunk_ld + j] *
  * 65536 (chunk_ld: at least the chunks of every tile). `tile_rows`: at least the rows of

@@ -630,12 +630,15 @@ lse_tmem_kernel(const float* __restrict__ src, const float* __restrict__ src2, c
 // against 31.2, 200 regions 105.0 against 105.2): their registers spill. Bulk copies of a row (512
 // bytes) take 100 cycles each (156 us); three loader warps have too few copies in flight (88 us).
 //
-// NP parts per operand: 1 single bf16, 2 split (hi, lo), 3 for the plain FP32 form (hi, mid, lo:
-// 24 bits; the six products down to 2^-18, smallest first, then hi * hi alone truncates). With
+// NP parts per operand: 1 single bf16, 2 split (hi, lo), 3 (hi, mid, lo: 24 bits; the six products
+// down to 2^-18, smallest first, then hi * hi alone truncates). Three parts are not FP32 arithmetic:
+// the truncation leaves a mean error of -1.6e-7 in the log values (FFMA with rounding: -2e-8), and
+// of an exponential below e^-75 the low part falls under bf16's subnormals (2^-18 of the value
+// left at e^-80, 2^-13 at e^-84, nothing below e^-87). So callers choose this form, it is no default. With
 // three parts A has one slot, D's two hold one chunk, whose sums go to shared memory when another
 // follows, and the weights then have one slot too. 119 tiles of 128 x
-// 128, batch 512, FP32: 40 us with the pack against 102 us for FFMA; error against FP64 no larger
-// (element flows 3.04e-7 against 3.06e-7).
+// 128, batch 512: 40 us with the pack against 102 us for FFMA; norm of the element flows' error
+// 3.04e-7 against 3.06e-7.
 constexpr int kPWarps = 16;
 constexpr int kPThreads = 32 * kPWarps + 32;
 constexpr int PT = KT / 4;  // terms per thread and chunk

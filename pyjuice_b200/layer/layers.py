@@ -135,7 +135,7 @@ _PACK3_BYTES = 98304  # the same weights in three bf16 parts (pcb_pack_weights_f
 
 
 def _pack3(holder: dict, table: torch.Tensor) -> torch.Tensor:
-    """The three-part packs of a tile or chunk table (FP32 form), allocated on the device at first
+    """The packs of a tile or chunk table for ``SumLayer.fp32_parts``, allocated on the device at first
     use; tied layers hold one buffer (``holder["pack3_of"]``, set by the circuit)."""
     h = holder.get("pack3_of") or holder
     if h.get("pack3") is None:
@@ -579,6 +579,14 @@ class SumLayer(Layer):
     # contractions with the samples along the tensor-memory lanes (pcb_lse_contract_tmem): None
     # autotuned against the others, False off, a number that ksplit (0: persistent)
     tmem = None
+    # Plain FP32 contractions of large layers on the tensor cores (see _f32_tmem for which, and for the
+    # times), a form that a caller asks for: its operands are three bf16 parts, not FP32. The tensor
+    # core truncates its sums (mean error of the log values -1.6e-7, of FP32 arithmetic -2e-8), and
+    # terms more than about 75 nats below the largest of their tile lose bits (2^-18 of their value
+    # at 80 nats, 2^-13 at 84, nothing left from 87 on), which counts where the larger terms have
+    # weight zero. Its packs hold 12 bytes per weight for the forward and as much again for the
+    # element flows.
+    fp32_parts = False
     # node flows x samples from which a backward that may not modify the flows writes log f -
     # log m to a workspace first (measured, us with / without: 200 regions of 256 x 256, batch 512:
     # 297 / 447; 119 of 128 x 128: 87 / 95; 25 of 128 x 128: 50 / 37, bound by the host)
@@ -806,8 +814,8 @@ class SumLayer(Layer):
 
     @staticmethod
     def _f32_tmem(tiles, tile_rows, max_terms, table, B):
-        """Whether an FP32 contraction runs on the tensor cores in three bf16 parts (the persistent
-        pcb_lse_contract_tmem): tiles of at least 64 rows and terms, and a (tile, 128-sample
+        """Whether an FP32 contraction is one that gains from three bf16 parts on the tensor cores (the
+        persistent pcb_lse_contract_tmem; taken with ``SumLayer.fp32_parts``): tiles of at least 64 rows and terms, and a (tile, 128-sample
         slice) for every other SM. Measured, forward with the pack against FFMA (us, batch 512):
         200 regions of 256 x 256: 179 / 773; 119 of 128 x 128: 40 / 102; 40 of 64 x 512: 44 / 84; 25
         of 96 x 96: 11.6 / 18.6; 100 of 32 x 32: 18.7 / 13.1."""
@@ -821,6 +829,13 @@ class SumLayer(Layer):
 
     def _el_f32(self, eg, B):
         return self._f32_tmem(eg["tiles"], eg["tm"], eg["max_terms"], eg["tiles"] if eg["short"] else eg["ch"], B)
+
+    def _fw_parts(self, d, prec, B):
+        """Whether the forward runs the three-part FP32 form."""
+        return prec == 0 and SumLayer.fp32_parts and self._fw_f32(d, B)
+
+    def _el_parts(self, eg, prec, B):
+        return prec == 0 and SumLayer.fp32_parts and self._el_f32(eg, B)
 
     @staticmethod
     def _run_f32(holder, tiles, tile_rows, table, index, src, aux, out, ld, B, krow, mode):
@@ -840,8 +855,8 @@ class SumLayer(Layer):
             return False
         if not backward:
             prec, tc05 = self._fw_tc05(d, B, force_use_bf16, force_use_fp32)
-            return d["fw_short"] and not tc05 and not (prec == 0 and self._fw_f32(d, B))
-        # (the FP32 form on the tensor cores takes rewritten flows, which are never fused)
+            return d["fw_short"] and not tc05 and not self._fw_parts(d, prec, B)
+        # (the three-part FP32 form takes rewritten flows, which are never fused)
         return all(eg["short"] and not self._el_tc05(eg, self._el_prec(eg, B, force_use_fp32))
                    for eg in d["el_groups"])
 
@@ -856,7 +871,7 @@ class SumLayer(Layer):
             return (d["fw_tiles"], d["kw"], d["fw_pack"], self.block_size, 1, 1 if (tc05 and prec == 3) else 0)
         if self._fw_long(d, prec):
             return (d["fw_ch"], d["kw"], _ch_pack(d, "fw_ch_pack"), self.block_size, 1, 1 if prec == 3 else 0)
-        if prec == 0 and self._fw_f32(d, B):
+        if self._fw_parts(d, prec, B):
             table = d["fw_tiles"] if d["fw_short"] else d["fw_ch"]
             return (table, d["kw"], _pack3(d["fw_f32"], table), self.block_size, 1, 2)
         return None
@@ -873,7 +888,7 @@ class SumLayer(Layer):
                              1 if (tc05 and prec == 3) else 0))
             elif self._el_long(eg, prec):
                 jobs.append((eg["ch"], eg["kw"], _ch_pack(eg, "ch_pack"), eg["cbs"], self.block_size, 1 if prec == 3 else 0))
-            elif prec == 0 and self._el_f32(eg, B):
+            elif self._el_parts(eg, prec, B):
                 table = eg["tiles"] if eg["short"] else eg["ch"]
                 jobs.append((table, eg["kw"], _pack3(eg, table), eg["cbs"], self.block_size, 2))
         return jobs
@@ -966,7 +981,7 @@ class SumLayer(Layer):
                        d["fw_ch_ranges"], d["krow"], 0, prec, st, holder=d, plan_key="fw_ch_plan", tiles=t,
                        tile_rows=d["fw_tm"], index=d["fw_ch_index"])
             return
-        if prec == 0 and kwargs.get("_fuse_fw") is None and self._fw_f32(d, B):
+        if kwargs.get("_fuse_fw") is None and self._fw_parts(d, prec, B):
             if not _weights_packed:
                 self.pack_forward_weights(params, B, force_use_bf16, force_use_fp32)
             short = d["fw_short"]
@@ -1033,7 +1048,7 @@ class SumLayer(Layer):
 
         def packed_form(eg):  # runs on the kernels that read packed weights
             p = self._el_prec(eg, B, force_use_fp32)
-            return self._el_tc05(eg, p) or self._el_long(eg, p) or (p == 0 and self._el_f32(eg, B))
+            return self._el_tc05(eg, p) or self._el_long(eg, p) or self._el_parts(eg, p, B)
 
         if (not allow_modify_flows and kwargs.get("_pflow_stream") is None and kwargs.get("_fuse_bw") is None
                 and (force_use_fp32 or SumLayer.bf16_form != 3)
@@ -1059,7 +1074,7 @@ class SumLayer(Layer):
             ready.record()
         # element flows
         if not _weights_packed and any(self._el_tc05(eg, p) or self._el_long(eg, p) or
-                                       (p == 0 and modified and self._el_f32(eg, B))
+                                       (modified and self._el_parts(eg, p, B))
                                        for eg in d["el_groups"] for p in (self._el_prec(eg, B, force_use_fp32),)):
             self.pack_flow_weights(params, B, force_use_fp32)
             _weights_packed = True
@@ -1077,7 +1092,7 @@ class SumLayer(Layer):
                            prec, nat.stream(), holder=eg, plan_key="ch_plan", tiles=et, tile_rows=eg["tm"],
                            index=eg["ch_index"])
                 continue
-            if prec == 0 and modified and self._el_f32(eg, B):
+            if modified and self._el_parts(eg, prec, B):
                 short = eg["short"]
                 self._run_f32(eg, et, eg["tm"], et if short else eg["ch"], None if short else eg["ch_index"], flows,
                               element_mars, element_flows, ld, B, eg["krow"], 1)

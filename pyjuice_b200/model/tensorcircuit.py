@@ -591,14 +591,20 @@ class TensorCircuit(nn.Module):
         (forward tiles, forward 128-term chunks, element-flow tiles and chunks), so the layers
         sharing a buffer also make the same kernel choices; the pack jobs then name the
         buffer once (``_multi_pack`` drops repeated buffers)."""
-        key = (self.device.type, self.device.index)
+        key = (self.device.type, self.device.index, SumLayer.fp32_parts)
         done = self.__dict__.setdefault("_shared_packs_done", set())
         if key in done or not TensorCircuit.share_tied_packs:
             return
         done.add(key)
-        canon = dict()
+        canon, contents = dict(), dict()
 
         def content(tiles, kw):
+            at = (tiles.data_ptr(), kw.data_ptr())
+            if at not in contents:  # once for all roles of a table
+                contents[at] = digest(tiles, kw)
+            return contents[at]
+
+        def digest(tiles, kw):
             t = tiles.cpu().numpy().astype(np.int64)
             kwn = kw.cpu().numpy()
             if t.shape[0] == 0:
@@ -624,7 +630,9 @@ class TensorCircuit(nn.Module):
             fh, fk, flazy = first
             holder[pack_key] = _ch_pack(fh, fk) if flazy else fh[fk]
 
-        def share3(role, holder, table, rpb, w_stride, kw):  # the FP32 form's packs, made on demand
+        def share3(role, holder, table, rpb, w_stride, kw):  # packs of the three-part form, made on demand
+            if not SumLayer.fp32_parts:
+                return
             c = None if table is None else content(table, kw)
             if c is not None:
                 first = canon.setdefault((role, rpb, w_stride) + c, holder)
@@ -730,7 +738,8 @@ class TensorCircuit(nn.Module):
         """What the element-flow packs depend on: the parameter values (storage, torch version
         counter, in-library writes) and the settings that select the packed layers."""
         return (self.params.data_ptr(), self.params._version, self._param_epoch, B, bool(force_use_fp32),
-                SumLayer.bf16_form, SumLayer.pack_short_weights, SumLayer.tc05_min_tiles, SumLayer.tmem is not False)
+                SumLayer.bf16_form, SumLayer.pack_short_weights, SumLayer.tc05_min_tiles, SumLayer.tmem is not False,
+                SumLayer.fp32_parts)
 
     # The forward of the run of small levels next to the root (product layer fused into the
     # single-stage sum kernel above it) in one persistent launch (pcb_lse_levels_short)

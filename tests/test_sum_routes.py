@@ -1,0 +1,50 @@
+"""Which entry points a sum layer calls, and which calls it refuses before any launch: the host
+side alone, with the launches recorded instead of made."""
+
+import pytest
+import torch
+
+import pyjuice_b200 as juice
+from pyjuice_b200 import _native as nat
+from pyjuice_b200.layer import layers as mod
+from pyjuice_b200.layer.layers import SumLayer
+from pyjuice_b200.nodes.distributions import Categorical
+
+
+@pytest.fixture
+def calls(monkeypatch):
+    """The entry points called, in order."""
+    names = []
+    monkeypatch.setattr(nat, "call", lambda name, *args: names.append(name))
+    monkeypatch.setattr(nat, "stream", lambda: None)
+    monkeypatch.setattr(nat, "ptr", lambda t: None)
+    monkeypatch.setattr(mod, "_num_sms", lambda: 148)
+    return names
+
+
+def _layer(regions, nodes, terms, bs):
+    with juice.set_block_size(bs):
+        leaves = [juice.inputs(v, num_node_blocks=terms // bs, dist=Categorical(num_cats=2)) for v in range(2 * regions)]
+        prods = [juice.multiply(leaves[2 * r], leaves[2 * r + 1]) for r in range(regions)]
+        sums = [juice.summate(p, num_node_blocks=nodes // bs) for p in prods]
+    juice.InputLayer(leaves, cum_nodes=bs)
+    juice.ProdLayer(prods)
+    return juice.SumLayer(sums, global_nid_start=bs, global_pid_start=bs ** 2, global_pfid_start=0, node2tiednodes=dict())
+
+
+def _buffers(layer, B, ld=None):
+    """Node values, node flows, element values, element flows: B columns of rows ``ld`` apart."""
+    rows = layer._layer_nid_range[1], max(int(c.max()) for c in layer.partitioned_chids) + 128
+    return [torch.zeros([n, ld or B])[:, :B] for n in (rows[0], rows[0], rows[1], rows[1])]
+
+
+@pytest.mark.parametrize("nodes,terms,B", [(128, 128, 512), (64, 272, 260), (96, 96, 8)])
+def test_plain_fp32_arithmetic(nodes, terms, B, calls):
+    """force_use_fp32, and batches below 16, take the FP32 kernels whatever the layer's size."""
+    layer = _layer(100, nodes, terms, 32 if terms % 32 == 0 else 16)
+    nm, nf, em, ef = _buffers(layer, B)
+    params = torch.zeros([1])
+    layer(nm, em, params, force_use_fp32=B >= 16)
+    for modify in (False, True):
+        layer.backward(nf, ef, nm, em, params, None, allow_modify_flows=modify, force_use_fp32=B >= 16)
+    assert set(calls) <= {"pcb_lse_contract", "pcb_lse_contract_short", "pcb_modify_flows"}
