@@ -1030,6 +1030,8 @@ class SumLayer(Layer):
         for t in (node_flows, element_flows, element_mars):
             if t.stride(0) != ld or t.stride(1) != 1:
                 raise ValueError("node/element mars/flows must share a row-major layout")
+            if t.size(1) < B:  # the kernels would read or write past its last row
+                raise ValueError("node/element mars/flows must have a column for every sample")
         if propagation_alg != "LL" or logspace_flows or negate_pflows or accumulate_ch_flows or allow_neg_flows:
             if allow_modify_flows:
                 raise ValueError("these flow modes read unmodified node flows: pass allow_modify_flows=False")
@@ -1041,6 +1043,8 @@ class SumLayer(Layer):
             self._backward_partial(part, node_flows, element_flows, node_mars, element_mars, params, param_flows,
                                    force_use_fp32)
             return
+        if param_flows is not None and (node_flows.size(1) != B or element_mars.size(1) != B):
+            raise ValueError("node flows, node values and element values must share one [rows, B] layout")
         if allow_modify_flows and not kwargs.get("_flows_modified"):
             nat.call("pcb_modify_flows", nat.ptr(node_flows), nat.ptr(node_mars), ld, B, self._layer_nid_range[0],
                      self._layer_nid_range[1], nat.stream())

@@ -48,3 +48,27 @@ def test_plain_fp32_arithmetic(nodes, terms, B, calls):
     for modify in (False, True):
         layer.backward(nf, ef, nm, em, params, None, allow_modify_flows=modify, force_use_fp32=B >= 16)
     assert set(calls) <= {"pcb_lse_contract", "pcb_lse_contract_short", "pcb_modify_flows"}
+
+
+@pytest.mark.parametrize("which", [1, 2, 3])
+@pytest.mark.parametrize("cut", [slice(8, None), slice(None, -8)])
+def test_backward_refuses_other_widths(which, cut, calls):
+    """Flows or values with other columns than the node values (same row stride) are refused before
+    the first launch, where there are too few of them and, once parameter flows are summed over
+    them, also where there are more; without parameter flows wider buffers serve as before."""
+    layer = _layer(4, 64, 64, 32)
+    bufs = _buffers(layer, 64, ld=72)
+    narrow = list(bufs)
+    narrow[which] = narrow[which][:, cut]
+    order = lambda b: (b[1], b[3], b[0], b[2], torch.zeros([1]))
+    pf = torch.zeros([1])
+    for flows in (None, pf):
+        with pytest.raises(ValueError):
+            layer.backward(*order(narrow), flows)
+    wide = [b if i == which else b[:, cut] for i, b in enumerate(bufs)]
+    if which != 3:
+        with pytest.raises(ValueError):
+            layer.backward(*order(wide), pf)
+    assert calls == []
+    layer.backward(*order(wide), None)
+    assert calls != []
