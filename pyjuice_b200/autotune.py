@@ -43,12 +43,18 @@ class Autotuner:
         return "|".join(map(str, key))
 
     def pick(self, key: Sequence[Hashable], candidates: Sequence, run: Callable[[object], None]):
-        """The chosen candidate for ``key`` (timing ``run(candidate)`` for each candidate on the
+        """The chosen candidate for ``key``, always one of ``candidates`` (timing ``run(candidate)`` for each candidate on the
         first eager call). ``run`` must launch on the current stream and leave its outputs
         equal for every candidate, or write them to scratch."""
         k = self._key(key)
         if k in self.choices:
-            return self.choices[k]
+            if self.choices[k] in candidates:
+                return self.choices[k]
+            # Kept by a call that had other forms on offer (alignment, settings): this set of them
+            # has a choice of its own.
+            k = self._key((k, "among") + tuple(candidates))
+            if self.choices.get(k) in candidates:
+                return self.choices[k]
         if not self.enabled or len(candidates) == 1:
             return candidates[0]
         if torch.cuda.is_current_stream_capturing():
