@@ -574,6 +574,7 @@ class SumLayer(Layer):
     bf16_form = 2
     short_kernels = True  # single-stage kernels for tiles of <= 128 terms
     tc05_min_tiles = 6    # layers with at least this many tiles use the tcgen05 kernels (BF16 forms)
+    tc05_min_chunks = 2   # long tiles of at least this many 128-term chunks use the tensor-memory form
     tc05_slices_per_cta = None  # sample slices per tcgen05 CTA (None: one)
     tc05_ws = None        # persistent warp-specialised tcgen05 kernel: None autotuned, True forced, False off
     # contractions with the samples along the tensor-memory lanes (pcb_lse_contract_tmem): None
@@ -807,10 +808,12 @@ class SumLayer(Layer):
 
     @staticmethod
     def _enough_chunks(ch, prec):
-        """Long tiles run on tcgen05 from two 128-term chunks on (at the default tc05_min_tiles): the
-        chunks run side by side where the mma.sync kernel walks them (figures at _tc05_long). E4M3, which rounds more than
-        that kernel, from tc05_min_tiles."""
-        return (1 if prec == 3 else 3) * ch.size(0) >= SumLayer.tc05_min_tiles
+        """Long tiles run on the tensor-memory form from tc05_min_chunks 128-term chunks on: the chunks
+        run side by side where the mma.sync kernel walks them (figures at _tc05_long). Without that
+        form the chunks are launches of their own and a combination, which pays from tc05_min_tiles
+        on; so does E4M3, which rounds more than the mma.sync kernel."""
+        return ch.size(0) >= (SumLayer.tc05_min_tiles if prec == 3 or SumLayer.tmem is False
+                              else SumLayer.tc05_min_chunks)
 
     @staticmethod
     def _f32_tmem(tiles, tile_rows, max_terms, table, B):

@@ -738,8 +738,8 @@ class TensorCircuit(nn.Module):
         """What the element-flow packs depend on: the parameter values (storage, torch version
         counter, in-library writes) and the settings that select the packed layers."""
         return (self.params.data_ptr(), self.params._version, self._param_epoch, B, bool(force_use_fp32),
-                SumLayer.bf16_form, SumLayer.pack_short_weights, SumLayer.tc05_min_tiles, SumLayer.tmem is not False,
-                SumLayer.fp32_parts)
+                SumLayer.bf16_form, SumLayer.pack_short_weights, SumLayer.tc05_min_tiles, SumLayer.tc05_min_chunks,
+                SumLayer.tc05_long, SumLayer.tmem is not False, SumLayer.fp32_parts)
 
     # The forward of the run of small levels next to the root (product layer fused into the
     # single-stage sum kernel above it) in one persistent launch (pcb_lse_levels_short)

@@ -72,3 +72,29 @@ def test_backward_refuses_other_widths(which, cut, calls):
     assert calls == []
     layer.backward(*order(wide), None)
     assert calls != []
+
+
+@pytest.mark.parametrize("nodes,terms", [(160, 160), (256, 256), (64, 320), (1024, 1024)])
+def test_without_the_tensor_memory_form(nodes, terms, calls, monkeypatch):
+    """``SumLayer.tmem = False`` brings back the kernels that long tiles had without it: mma.sync
+    below tc05_min_tiles chunks, chunk launches from there on."""
+    layer = _layer(1, nodes, terms, 32)
+    nm, nf, em, ef = _buffers(layer, 64)
+    params = torch.zeros([1])
+    forward, flows = ({"pcb_lse_contract"} if tiles * -(-k // 128) < 6 else {"pcb_pack_weights", "chunks"}
+                      for tiles, k in ((-(-nodes // 128), terms), (-(-terms // 128), nodes)))
+    chunk_forms = {"pcb_lse_contract_tc05", "pcb_lse_contract_tc05_ws", "pcb_lse_contract_tc05_accum", "pcb_chunk_combine"}
+    monkeypatch.setattr(mod.TUNER, "enabled", False)
+    for tmem in (False, None):
+        monkeypatch.setattr(SumLayer, "tmem", tmem)
+        for run, want in ((lambda: layer(nm, em, params, force_use_bf16=True), forward),
+                          (lambda: layer.backward(nf, ef, nm, em, params, None, allow_modify_flows=True,
+                                                  _flows_modified=True), flows)):
+            calls.clear()
+            run()
+            got = {"chunks" if c in chunk_forms else c for c in calls}
+            if tmem is False:
+                short = want is flows and nodes <= 128  # flows of few nodes: short tiles
+                assert got == ({"pcb_lse_contract_short"} if short else want)
+            else:
+                assert "pcb_lse_contract" not in got
