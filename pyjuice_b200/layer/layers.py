@@ -149,10 +149,13 @@ kTmemCluster = 8  # most CTAs that share a tile in pcb_lse_contract_tmem
 def _tmem_ksplit(num_tiles: int, tile_rows: int, num_chunks: int, B: int) -> int:
     """CTAs (a cluster) that share a tile's chunks in pcb_lse_contract_tmem (``ksplit``). Tiles
     of more than 64 rows: one per chunk, so that two CTAs fit on an SM (the sums of several
-    chunks take another 64 KB of shared memory); lower tiles: as many as still run at once."""
+    chunks take another 64 KB of shared memory) and none is without a chunk; lower tiles: as many
+    as still run at once. Measured with one CTA per chunk against eight (us, forward, graph-timed):
+    768 x 768, batch 64: 9.6 / 10.4, batch 512: 13.6 / 14.7; four of them, batch 512: 34.8 / 43.2; 896 x
+    896, batch 64: 10.5 / 10.7; four of them, batch 512: 47.7 / 52.2."""
     if tile_rows > 64:
-        return num_chunks if num_chunks < 6 else 8
-    return max(1, min(8, num_chunks, 2 * _num_sms() // (num_tiles * -(-B // 128))))
+        return min(kTmemCluster, num_chunks)
+    return max(1, min(kTmemCluster, num_chunks, 2 * _num_sms() // (num_tiles * -(-B // 128))))
 
 
 def _tmem_pays(sub_tiles: int, B: int) -> bool:

@@ -98,3 +98,13 @@ def test_without_the_tensor_memory_form(nodes, terms, calls, monkeypatch):
                 assert got == ({"pcb_lse_contract_short"} if short else want)
             else:
                 assert "pcb_lse_contract" not in got
+
+
+@pytest.mark.parametrize("chunks", range(1, 20))
+@pytest.mark.parametrize("tiles,rows,B", [(1, 128, 64), (6, 128, 512), (200, 128, 512), (1, 64, 64), (40, 32, 200)])
+def test_every_cta_of_a_cluster_has_a_chunk(chunks, tiles, rows, B, monkeypatch):
+    monkeypatch.setattr(mod, "_num_sms", lambda: 148)
+    ks = mod._tmem_ksplit(tiles, rows, chunks, B)
+    assert 1 <= ks <= min(chunks, mod.kTmemCluster)
+    # one each as long as a cluster has a CTA per chunk (taller tiles need the shared memory)
+    assert rows <= 64 or ks == min(chunks, mod.kTmemCluster)
