@@ -31,6 +31,11 @@ from ..layer.layers import InputLayer, LayerGroup, ProdLayer, SumLayer, _ch_pack
 from ..nodes import CircuitNodes, multiply, summate
 
 
+# Whether a tensor is a functorch wrapper, whose values no kernel can read (None: this torch
+# does not tell)
+_is_wrapped = getattr(getattr(torch._C, "_functorch", None), "is_functorch_wrapped_tensor", None)
+
+
 def _pc_model_backward_hook(grad, pc, inputs, record_cudagraph, apply_cudagraph, propagation_alg, **kwargs):
     """Gradient hook on the returned log-likelihoods (tensorcircuit.py:24-37).
 
@@ -1198,7 +1203,7 @@ class TensorCircuit(nn.Module):
                 type(grad) is torch.Tensor and nf is not None and grad.layout == torch.strided and
                 grad.dtype == torch.float32 and grad.device == nf.device and
                 grad.shape == (nf.size(1), self.num_root_nodes) and 0 < grad.numel() <= (1 << 14) and
-                not grad.is_neg() and not torch._C._functorch.is_functorch_wrapped_tensor(grad))
+                not grad.is_neg() and _is_wrapped is not None and not _is_wrapped(grad))
 
     @property
     def _cum_flow(self) -> float:
