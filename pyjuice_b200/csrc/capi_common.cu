@@ -40,6 +40,7 @@ namespace {
 __device__ int32_t g_status_word = 0;
 constexpr int kMaxDevices = 64;
 std::atomic<int32_t*> g_status_addr[kMaxDevices];
+std::atomic<int> g_num_sms[kMaxDevices];
 }  // namespace
 
 int32_t* status_word() {
@@ -56,6 +57,21 @@ int32_t* status_word() {
         g_status_addr[dev].store(p, std::memory_order_release);
     }
     return p;
+}
+
+int num_sms() {
+    constexpr int kB200 = 148;
+    int dev = 0, n = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return kB200;
+    n = g_num_sms[dev].load(std::memory_order_relaxed);
+    if (n == 0) {
+        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) {
+            cudaGetLastError();
+            return kB200;
+        }
+        g_num_sms[dev].store(n, std::memory_order_relaxed);
+    }
+    return n;
 }
 
 int check_launch(const char* what) {

@@ -150,6 +150,9 @@ int launch_status(cudaError_t e, const char* what);
 // PCB_STATUS_* bits into it when they detect a fault; pcb_device_status reads it.
 int32_t* status_word();
 
+// SMs of the current device (asked once per device; the B200's 148 if the look-up fails).
+int num_sms();
+
 __device__ __forceinline__ void report_status(int32_t* status, int32_t bits) {
     if (status) atomicOr(status, bits);
 }

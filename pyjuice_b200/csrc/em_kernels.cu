@@ -269,7 +269,7 @@ int input_em_launch(float* params, const FT* param_flows, const int32_t* s_pids,
     if (!(step_size > 0.0 && step_size <= 1.0)) return pcb::set_error(PCB_E_ARG, "%s: step_size must be in (0, 1]", name);
     if (num_source_nodes == 0) return PCB_OK;
     // several nodes per warp only once that leaves 16 warps per SM
-    const int npw = (int)std::max<int64_t>(1, std::min<int64_t>(kEmNodes, num_source_nodes / (148 * 16)));
+    const int npw = (int)std::max<int64_t>(1, std::min<int64_t>(kEmNodes, num_source_nodes / (pcb::num_sms() * 16)));
     const unsigned grid = (unsigned)pcb::cdiv(pcb::cdiv(num_source_nodes, npw) * 32, 256);
     cudaStream_t s = pcb::as_stream(stream);
     if (keep_zero_params) {

@@ -407,7 +407,8 @@ extern "C" int pcb_input_cat_bwd(const int64_t* data, int64_t data_ld, const flo
         return pcb::set_error(PCB_E_ARG, "pcb_input_cat_bwd: bad arguments");
     if (num_groups == 0) return PCB_OK;
     const int CB = B < kBwChunk ? B : kBwChunk;
-    // the supported range: vocabularies of up to about 50,000 categories
+    // The range that this entry has always taken, by batch size: 39,933 categories from a batch of
+    // 1024 on, 48,381 at 256 (this kernel's own tables stop growing at 510 categories).
     if (((int64_t)11 * std::min(B, 1024) + max_ncats + 3) * (int64_t)sizeof(int) > 200 * 1024)
         return pcb::set_error(PCB_E_ARG, "pcb_input_cat_bwd: too many categories (%d)", max_ncats);
     const size_t smem = BwdSmem(CB, max_ncats).total;
@@ -418,7 +419,7 @@ extern "C" int pcb_input_cat_bwd(const int64_t* data, int64_t data_ld, const flo
         }
         // CTAs per variable: one where the variables alone give three per SM (each sorts the
         // batch again), up to 16 for fewer; a CTA without a tile returns at once
-        const int splits = (int)std::min<int64_t>(16, pcb::cdiv(3 * 148, num_groups));
+        const int splits = (int)std::min<int64_t>(16, pcb::cdiv(3 * pcb::num_sms(), num_groups));
         return pcb::launch_status(pcb::launch_k(kernel, dim3(num_groups, splits), dim3(32 * kBwWarps), smem,
                                                 pcb::as_stream(stream), 1u, data, data_ld, node_flows, ld, B, grp_var,
                                                 grp_node0, grp_count, grp_ncats, s_pfids, node_offset, param_flows,

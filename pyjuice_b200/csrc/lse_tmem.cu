@@ -1105,14 +1105,12 @@ int launch_persistent(const float* src, const float* src2, const float* aux, flo
     }
     const size_t smem = S.total;
     static bool configured[64] = {false};
-    static int sms[64] = {0};
     int dev = 0;
     cudaGetDevice(&dev);
     dev = dev < 0 ? 0 : (dev > 63 ? 63 : dev);
     if (!configured[dev]) {
         cudaError_t e = cudaFuncSetAttribute(lse_tmem_persistent_kernel<MODE, NP, COPY>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms[dev], cudaDevAttrMultiProcessorCount, dev);
         if (e != cudaSuccess) return pcb::set_error(PCB_E_CUDA, "pcb_lse_contract_tmem: %s", cudaGetErrorString(e));
         configured[dev] = true;
     }
@@ -1120,7 +1118,7 @@ int launch_persistent(const float* src, const float* src2, const float* aux, flo
     const int64_t units = (int64_t)num_tiles * slices;
     if (units > INT32_MAX) return pcb::set_error(PCB_E_ARG, "pcb_lse_contract_tmem: too many tiles");
     return pcb::launch_status(
-        pcb::launch_k(lse_tmem_persistent_kernel<MODE, NP, COPY>, dim3((unsigned)std::min<int64_t>(units, sms[dev])),
+        pcb::launch_k(lse_tmem_persistent_kernel<MODE, NP, COPY>, dim3((unsigned)std::min<int64_t>(units, pcb::num_sms())),
                       dim3(kPThreads), smem, s, 1u, src, src2, aux, out, ld, B, packed, tiles, krow, chunk_index,
                       chunk_ld, n_max, sums, slices, (int)units, pcb::status_word()),
         "pcb_lse_contract_tmem");

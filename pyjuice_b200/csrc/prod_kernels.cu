@@ -155,7 +155,7 @@ int launch_prod(const char* name, const float* in, float* out, int64_t ld, int32
     const bool vec = pcb::vec_ok(in, ld) && pcb::vec_ok(out, ld) && (!MOD || pcb::vec_ok(nm, ld));
     const int ngrp = (int)(vec ? pcb::cdiv(B, 4) : 32 * pcb::cdiv(B, 128));
     // Four rows per thread once that still leaves two full sets of threads per SM.
-    const bool wide = !LSE && blk_size >= 4 && (int64_t)num_blocks * blk_size / 4 * ngrp >= 2LL * 148 * 2048;
+    const bool wide = !LSE && blk_size >= 4 && (int64_t)num_blocks * blk_size / 4 * ngrp >= 2LL * pcb::num_sms() * 2048;
     const int rows = wide ? 4 : 1;
     const int per_blk = (int)pcb::cdiv(blk_size, rows);
     const int64_t chunks = (int64_t)num_blocks * per_blk;
