@@ -45,12 +45,6 @@ struct Plan {
     static constexpr size_t bytes() { return oSlot + 16; }
 };
 
-__device__ __forceinline__ float ex2(float x) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-
 // D f32, A and B bf16, both MN-major, M = 128, N
 template <int N>
 __device__ __forceinline__ constexpr uint32_t idesc_mn() {

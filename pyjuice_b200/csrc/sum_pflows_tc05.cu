@@ -37,12 +37,6 @@ constexpr float kLog2e = 1.4426950408889634f;
 constexpr uint32_t kLBO = 128;            // core matrices adjacent along K
 constexpr uint32_t kSBO = (KB / 8) * 128;  // 8-row groups
 
-__device__ __forceinline__ float ex2(float x) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-
 // byte offset of (row r, sample k) in a K-major operand of 32 samples
 __device__ __forceinline__ uint32_t op_off(int r, int k) {
     return (uint32_t)(r >> 3) * kSBO + (uint32_t)(k >> 3) * kLBO + (uint32_t)(r & 7) * 16 + (uint32_t)(k & 7) * 2;

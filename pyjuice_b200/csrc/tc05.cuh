@@ -63,6 +63,26 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* m, uint32_t parity) 
     return false;
 }
 
+// Bytes that the barrier's current phase still waits for (and the one arrival)
+__device__ __forceinline__ void mbar_expect_tx(uint64_t* m, uint32_t bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(smem_u32(m)), "r"(bytes) : "memory");
+}
+
+// Untiled bulk copy of this GPU's memory to shared memory (16-byte aligned, a multiple of 16 bytes)
+__device__ __forceinline__ void bulk_copy_g2s(void* dst, const void* src, uint32_t bytes, uint64_t* mbar) {
+    asm volatile(
+        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(
+            smem_u32(dst)),
+        "l"(src), "r"(bytes), "r"(smem_u32(mbar))
+        : "memory");
+}
+
+__device__ __forceinline__ float ex2(float x) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
 // An allocation waits, without a limit, until the SM has so many of its 512 columns free, so no
 // CTA that holds columns may wait for one that still allocates:
 // * A kernel lets its successor start (pdl_trigger) only after its own allocation, by the warp
