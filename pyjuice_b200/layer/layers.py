@@ -1063,6 +1063,7 @@ class SumLayer(Layer):
         if (not allow_modify_flows and kwargs.get("_pflow_stream") is None and kwargs.get("_fuse_bw") is None
                 and (force_use_fp32 or SumLayer.bf16_form != 3)
                 and (self._layer_nid_range[1] - self._layer_nid_range[0]) * B >= SumLayer.ratio_min_values
+                and ld <= 2 * B  # the workspace has the caller's row stride: not for a few columns of wide rows
                 and all(map(packed_form, d["el_groups"]))):
             # log f - log m of this layer's nodes once, in a workspace, instead of in every tile
             # of both contractions that reads them (node_flows stays as the caller has it)

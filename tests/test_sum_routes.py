@@ -108,3 +108,19 @@ def test_every_cta_of_a_cluster_has_a_chunk(chunks, tiles, rows, B, monkeypatch)
     assert 1 <= ks <= min(chunks, mod.kTmemCluster)
     # one each as long as a cluster has a CTA per chunk (taller tiles need the shared memory)
     assert rows <= 64 or ks == min(chunks, mod.kTmemCluster)
+
+
+@pytest.mark.parametrize("ld,taken", [(512, True), (1024, True), (1028, False), (8192, False)])
+def test_ratio_workspace_is_no_larger_than_the_flows(ld, taken, calls, monkeypatch):
+    """The workspace of log f - log m has the row stride of the caller's buffers, so a batch that is
+    a few columns of wide rows goes without it."""
+    layer = _layer(8, 128, 128, 32)
+    monkeypatch.setattr(SumLayer, "ratio_min_values", 0)
+    monkeypatch.setattr(mod.TUNER, "enabled", False)
+    buf = torch.empty([layer._layer_nid_range[1], ld])[:, :512]
+    made = []
+    empty = torch.empty
+    monkeypatch.setattr(mod.torch, "empty", lambda shape, **kw: (made.append(shape), empty([1, 1]))[1])
+    layer.backward(buf, buf, buf, buf, torch.zeros([1]), None)
+    assert ("pcb_flow_ratios" in calls) == taken
+    assert [s for s in made if list(s)[-1] == ld] == ([[8 * 128, ld]] if taken else [])
