@@ -889,7 +889,7 @@ def main():
         pf = pflows_roofline(pc)
         achieved = pf["bytes"] / pf["seconds"] / 1e9
         roof = {"kernel": "pcb_sum_pflows_lanes (autotuned, split-bf16 form, 64-child tiles) of the largest "
-                          "sum layer: the kernel with the largest share of the step",
+                          "sum layer: parameter flows are the pass with the largest share of the step",
                 "bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s", "frac": achieved / hbm,
                 "traffic": PFLOW_TRAFFIC_BYTES,
                 "traffic_source": "dram__bytes_read.sum + dram__bytes_write.sum of this launch, one ncu capture "
@@ -901,9 +901,9 @@ def main():
                                               "achieved_gbs": big["bytes"] / big["seconds"] / 1e9,
                                               "frac": big["bytes"] / big["seconds"] / 1e9 / hbm,
                                               "tiles": big["tiles"],
-                                              "kernel": "tcgen05 contraction (autotuned: persistent "
-                                                        "warp-specialised or CTA-per-slice), weights packed "
-                                                        "beforehand",
+                                              "kernel": "tcgen05 contraction (autotuned over the tensor-memory, "
+                                                        "warp-specialised and CTA-per-slice forms), weights "
+                                                        "packed beforehand",
                                               "pack_us": big["pack_seconds"] * 1e6},
                 "all_sum_layers_forward": {"layers": rf["layers"], "us_total": rf["seconds"] * 1e6,
                                            "achieved_gbs": rf["bytes"] / rf["seconds"] / 1e9,

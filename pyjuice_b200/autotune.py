@@ -2,9 +2,15 @@
 candidate launch shape is timed on the device and the fastest is kept for that key.
 
 Keys describe the work, not the layer: kernel family, mode, precision form, number of
-tiles, tallest tile, batch size (``SumLayer`` builds them). Candidates produce the same
-results (they only change how samples and tiles map to CTAs); accumulating launches are
-tuned on scratch buffers (the caller's ``run`` decides where a candidate writes). Timing
+tiles, tallest tile, batch size (``SumLayer`` builds them). Candidates compute the same sums
+within the same error bounds, but not all in the same order: contractions of long tiles (chunks
+combined in log space, cluster, persistent) and parameter flows (over how many parts of the batch
+they are summed apart) differ in their last bits. A choice rests on a
+timing, so those bits can differ between processes, and between the first eager pass and one
+captured before it. ``PCB_AUTOTUNE=0`` pins them (static defaults), as does a file of choices that
+every process reads; ``SumLayer.tmem``, ``pflow_tc05`` and ``pflow_tile_children`` name single forms.
+Accumulating launches are tuned on scratch buffers (the caller's ``run`` decides where a candidate
+writes). Timing
 uses CUDA events on the current stream: two warm-up runs per candidate, then the median of
 ``reps`` timed runs. Nothing is tuned while a CUDA graph is being captured: a key not yet
 tuned then takes the first candidate (the static default) and is tuned at its next eager
@@ -44,8 +50,8 @@ class Autotuner:
 
     def pick(self, key: Sequence[Hashable], candidates: Sequence, run: Callable[[object], None]):
         """The chosen candidate for ``key``, always one of ``candidates`` (timing ``run(candidate)`` for each candidate on the
-        first eager call). ``run`` must launch on the current stream and leave its outputs
-        equal for every candidate, or write them to scratch."""
+        first eager call). ``run`` must launch on the current stream and overwrite its
+        outputs, or write them to scratch."""
         k = self._key(key)
         if k in self.choices:
             if self.choices[k] in candidates:
