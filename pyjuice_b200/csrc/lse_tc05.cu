@@ -340,8 +340,8 @@ lse_tc05_kernel(const float* __restrict__ src, const float* __restrict__ src2, c
                 float* __restrict__ out, int64_t ld, int B, const uint8_t* __restrict__ packed,
                 const PcbLseTile* __restrict__ tiles, const int* __restrict__ krow, int spc, bool vec,
                 bool accum, int32_t* __restrict__ status) {
-    // tile and term indices (compiled tables) and the tensor memory before the wait for the
-    // previous kernel
+    // tile and term indices (compiled tables) before the wait for the previous kernel
+    pcb::pdl_trigger();
     static_assert(N == 32 || N == 64, "sample slice");
     constexpr bool SPLIT = PREC == 2;
     constexpr bool FP8 = PREC == 3;
@@ -370,9 +370,11 @@ lse_tc05_kernel(const float* __restrict__ src, const float* __restrict__ src2, c
     const int nk = bad ? 0 : t.k_cnt;
     const int s0 = blockIdx.y * spc;
     const int nsl = min(spc, (B + N - 1) / N - s0);
+    if (tid < nk) sRow[tid] = __ldg(krow + t.k_off + tid);
+    pcb::pdl_wait();
+
     if (warp == 0) {
         tmem_alloc(slot, N);
-        pcb::pdl_trigger();
         asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
     }
     if (tid == 0) {
@@ -381,11 +383,9 @@ lse_tc05_kernel(const float* __restrict__ src, const float* __restrict__ src2, c
         slot[1] = 0;
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
-    if (tid < nk) sRow[tid] = __ldg(krow + t.k_off + tid);
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
     const uint32_t taddr = slot[0];
-    pcb::pdl_wait();
     if (tid == 0) {
         const uint32_t wbytes = FP8 ? kF8TileBytes : (SPLIT ? kTileBytes : kHalfBytes);
         mbar_expect_tx(barW, wbytes);
@@ -758,6 +758,7 @@ lse_tc05_ws_kernel(const __grid_constant__ CUtensorMap map_src, const __grid_con
                    const __grid_constant__ CUtensorMap map_out, const float* __restrict__ aux, float* __restrict__ out, int64_t ld, int B, int run_log2,
                    const uint8_t* __restrict__ packed, const PcbLseTile* __restrict__ tiles, int num_tiles,
                    const int* __restrict__ krow, int32_t* __restrict__ status) {
+    pcb::pdl_trigger();
     static_assert(N == 32 || N == 64, "sample slice");
     using S = WsSmem<N, MODE, SPLIT>;
     constexpr int NS = S::NS;
@@ -786,7 +787,6 @@ lse_tc05_ws_kernel(const __grid_constant__ CUtensorMap map_src, const __grid_con
 
     if (warp == 1) {
         tmem_alloc(const_cast<uint32_t*>(slot), 2 * N);
-        pcb::pdl_trigger();
         asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
     }
     if (tid == 0) {

@@ -237,6 +237,7 @@ lse_tmem_kernel(const float* __restrict__ src, const float* __restrict__ src2, c
                 const PcbLseTile* __restrict__ tiles, const int* __restrict__ krow,
                 const int* __restrict__ chunk_index, int chunk_ld, int n_max, bool several,
                 int num_slices, int32_t* __restrict__ status) {
+    pcb::pdl_trigger();
     extern __shared__ __align__(1024) uint8_t sm[];
     cg::cluster_group cluster = cg::this_cluster();
     const int ks = (int)cluster.num_blocks();
@@ -265,7 +266,6 @@ lse_tmem_kernel(const float* __restrict__ src, const float* __restrict__ src2, c
 
     if (warp == 8) {
         tmem_alloc(slot, kCols);
-        pcb::pdl_trigger();
         fence_before_sync();
     }
     // the first chunk's source rows (compiled tables), the tile's first one beyond its terms
@@ -666,6 +666,7 @@ lse_tmem_persistent_kernel(const float* __restrict__ src, const float* __restric
                            const uint8_t* __restrict__ packed, const PcbLseTile* __restrict__ tiles,
                            const int* __restrict__ krow, const int* __restrict__ chunk_index, int chunk_ld, int n_max,
                            bool sums, int num_slices, int num_units, int32_t* __restrict__ status) {
+    pcb::pdl_trigger();
     extern __shared__ __align__(1024) uint8_t sm[];
     constexpr int AS = NP == 3 ? 1 : 2;  // slots of A
     static_assert(NP < 3 || MODE < 2, "the FP32 form takes rewritten flows");
@@ -686,7 +687,6 @@ lse_tmem_persistent_kernel(const float* __restrict__ src, const float* __restric
 
     if (warp == kPWarps) {
         tmem_alloc(slot, 512);
-        pcb::pdl_trigger();
         fence_before_sync();
     }
     if (tid == 0) {

@@ -82,6 +82,7 @@ sum_pflows_lanes_kernel(const float* __restrict__ nf, const float* __restrict__ 
                         int64_t ld, int B, const float* __restrict__ params, float* __restrict__ pf,
                         const PcbPflowTile* __restrict__ tiles, int rpb_log2, const int* __restrict__ cids,
                         const int* __restrict__ pids, const int* __restrict__ pfids, int32_t* __restrict__ status) {
+    pcb::pdl_trigger();
     using P = Plan<TKC>;
     constexpr int CP = TKC / 4;  // children per warp part
     extern __shared__ __align__(1024) uint8_t sm[];
@@ -95,16 +96,15 @@ sum_pflows_lanes_kernel(const float* __restrict__ nf, const float* __restrict__ 
     const PcbPflowTile t = tiles[blockIdx.x];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
-    if (warp == 0) {
-        tmem_alloc(slot, kCols);
-        pcb::pdl_trigger();
-        fence_before_sync();
-    }
     for (int i = tid; i < TKC; i += kThreads) {  // places beyond the children read the first one's row
         const int k = t.k_off + (i < t.k_cnt ? i : 0);
         sCid[i] = __ldg(cids + k);
         sPid[i] = __ldg(pids + k);
         sPfid[i] = __ldg(pfids + k);
+    }
+    if (warp == 0) {
+        tmem_alloc(slot, kCols);
+        fence_before_sync();
     }
     if (tid == 32) {
         mbar_init(bar, 1);

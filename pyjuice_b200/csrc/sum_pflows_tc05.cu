@@ -69,6 +69,7 @@ sum_pflows_tc05_kernel(const float* __restrict__ nf, const float* __restrict__ n
                        const PcbPflowTile* __restrict__ tiles, int rpb_log2, const int* __restrict__ cids,
                        const int* __restrict__ pids, const int* __restrict__ pfids, int slice, bool vec,
                        const int* __restrict__ deltas, int nlay, int32_t* __restrict__ status) {
+    pcb::pdl_trigger();
     using P = Plan<TKC, MODIFIED>;
     static_assert(TKC == 64 || TKC == 128, "children per tile");
     extern __shared__ __align__(1024) uint8_t smem[];
@@ -90,16 +91,15 @@ sum_pflows_tc05_kernel(const float* __restrict__ nf, const float* __restrict__ n
     const int lane = tid & 31;
     const int rpb_mask = (1 << rpb_log2) - 1;
 
-    if (warp == 0) {
-        tmem_alloc(slot, TKC);
-        pcb::pdl_trigger();
-        fence_before_sync();
-    }
     if (tid < TKC) {
         const bool in = tid < t.k_cnt;
         sCid[tid] = in ? __ldg(cids + t.k_off + tid) : -1;
         sPid[tid] = in ? __ldg(pids + t.k_off + tid) : 0;
         sPfid[tid] = in ? __ldg(pfids + t.k_off + tid) : 0;
+    }
+    if (warp == 0) {
+        tmem_alloc(slot, TKC);
+        fence_before_sync();
     }
     if (tid == 32) {
         mbar_init(&bar[0], 1);

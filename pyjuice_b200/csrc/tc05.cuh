@@ -83,15 +83,6 @@ __device__ __forceinline__ float ex2(float x) {
     return y;
 }
 
-// An allocation waits, without a limit, until the SM has so many of its 512 columns free, so no
-// CTA that holds columns may wait for one that still allocates:
-// * A kernel lets its successor start (pdl_trigger) only after its own allocation, by the warp
-//   that made it. A successor's CTA holds its columns through pdl_wait, that is until every CTA
-//   of this grid is done; had one of those not allocated yet, both would wait for good. All
-//   grids before it in the stream have their columns for the same reason.
-// * The CTAs of a cluster wait for one another with their columns held. Those of any two clusters
-//   that an SM's 227 KB of shared memory can take together fit in its columns: lse_tmem_kernel
-//   has 256 columns and at least 77 KB, sum_pflows_tc05_kernel at most 128 and at least 107 KB.
 __device__ __forceinline__ void tmem_alloc(uint32_t* slot, uint32_t ncols) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(slot)),
                  "r"(ncols)
