@@ -786,6 +786,7 @@ lse_tc05_ws_kernel(const __grid_constant__ CUtensorMap map_src, const __grid_con
     const int64_t u0 = units * blockIdx.x / gridDim.x, u1 = units * (blockIdx.x + 1) / gridDim.x;
 
     if (warp == 1) {
+        pcb::pdl_wait();
         tmem_alloc(const_cast<uint32_t*>(slot), 2 * N);
         asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
     }
@@ -1167,6 +1168,7 @@ int launch_ws(int num_tiles, int num_ctas, const CUtensorMap& m1, const CUtensor
               int64_t ld, int B, int run_log2, const uint8_t* packed, const PcbLseTile* tiles, const int* krow,
               cudaStream_t s) {
     constexpr size_t smem = WsSmem<N, MODE, SPLIT>::bytes();
+    static_assert(smem >= 80 * 1024, "what shares an SM must fit its tensor memory (tc05.cuh)");
     static_assert(smem <= 227 * 1024, "shared memory");
     static bool configured[64] = {false};
     const int dev = current_device();
@@ -1200,6 +1202,7 @@ template <int N, int MODE, int PREC>
 int launch(int num_tiles, int spc, const float* src, const float* src2, const float* aux, float* out, int64_t ld,
            int B, const uint8_t* packed, const PcbLseTile* tiles, const int* krow, cudaStream_t s, bool vec, bool accum) {
     constexpr size_t smem = Tc05Smem<N>::bytes();
+    static_assert(smem >= 80 * 1024, "what shares an SM must fit its tensor memory (tc05.cuh)");
     static_assert(smem <= 227 * 1024, "shared memory");
     static bool configured[64] = {false};
     const int dev = current_device();

@@ -60,6 +60,7 @@ constexpr uint32_t kLBO = 128;                 // bytes between core matrices al
 constexpr uint32_t kSBO = (KT / 8) * 128;      // bytes between 8-row groups
 constexpr uint32_t kColsD = 128, kColsA = KT / 2, kCols = 256;
 constexpr int kMaxCluster = 8;
+constexpr uint32_t kShared = 77 * 1024;        // least shared memory of a CTA
 
 struct Smem {
     // the weights come first (n_pad x 128 x (hi + lo) bf16), and in their place, once the MMAs
@@ -627,6 +628,7 @@ constexpr int kPThreads = 32 * kPWarps + 32;
 constexpr int PT = KT / 4;  // terms per thread and chunk
 constexpr int EB = 8;       // accumulator columns per epilogue step
 constexpr int kRowRing = 4;
+constexpr uint32_t kPShared = 152 * 1024;  // least shared memory of a CTA
 constexpr uint32_t kPSlots = 216 * 1024;  // shared memory for weights, sums and values
 
 struct PSmem {
@@ -685,10 +687,6 @@ lse_tmem_persistent_kernel(const float* __restrict__ src, const float* __restric
     const int u0 = (int)((int64_t)num_units * blockIdx.x / gridDim.x);
     const int u1 = (int)((int64_t)num_units * (blockIdx.x + 1) / gridDim.x);
 
-    if (warp == kPWarps) {
-        tmem_alloc(slot, 512);
-        fence_before_sync();
-    }
     if (tid == 0) {
         for (int i = 0; i < 2; ++i) {
             mbar_init(barW + i, 1);
@@ -701,8 +699,12 @@ lse_tmem_persistent_kernel(const float* __restrict__ src, const float* __restric
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
     __syncthreads();
-    fence_after_sync();
-    const uint32_t taddr = slot[0];
+    uint32_t taddr = 0;
+    auto columns = [slot]() {  // all warps, once warp 16 has allocated
+        asm volatile("bar.sync 2, %0;\n" ::"n"(kPThreads) : "memory");
+        fence_after_sync();
+        return *slot;
+    };
     // columns: D of slots 0 and 1, then A (its parts side by side) of slots 0 and 1
     auto d_cols = [&](int q) { return taddr + (NP == 3 ? 0 : (q & 1) * kColsD); };
     auto a_cols = [&](int q) { return taddr + 2 * kColsD + (AS == 1 ? 0 : (q & 1) * 2 * kColsA); };
@@ -752,6 +754,9 @@ lse_tmem_persistent_kernel(const float* __restrict__ src, const float* __restric
         put_rows();
         pcb::pdl_wait();
         if (S.nw == 2) copy_weights();
+        tmem_alloc(slot, 512);
+        fence_before_sync();
+        taddr = columns();
         int q = 0;
         for (int u = u0; u < u1; ++u) {
             const PcbLseTile t = tiles[u / num_slices];
@@ -938,6 +943,7 @@ lse_tmem_persistent_kernel(const float* __restrict__ src, const float* __restric
                 load(0, b0, nk, Z{});
             }
         }
+        taddr = columns();  // the first rows are already requested
         for (int u = u0; u < u1; ++u) {
             t = tiles[u / num_slices];
             const int nch = chunks_of(t);
@@ -1086,7 +1092,8 @@ int launch_persistent(const float* src, const float* src2, const float* aux, flo
             return launch_persistent<MODE, NP, false>(src, src2, aux, out, ld, B, packed, tiles, num_tiles, n_max, krow,
                                                       chunk_index, chunk_ld, s);
     }
-    const size_t smem = S.total;
+    // no CTA of the other form, which allocates early, beside this one (tc05.cuh)
+    const size_t smem = std::max<size_t>(S.total, kPShared);
     static bool configured[64] = {false};
     int dev = 0;
     cudaGetDevice(&dev);
@@ -1112,9 +1119,9 @@ int launch(const float* src, const float* src2, const float* aux, float* out, in
            const PcbLseTile* tiles, int num_tiles, int n_max, const int* krow, const int* chunk_index, int chunk_ld,
            int ksplit, cudaStream_t s) {
     const bool several = chunk_index && chunk_ld > ksplit;
-    // The CTAs of a cluster wait for one another with their tensor memory allocated, so never
-    // more of them than the tensor memory serves (two) may be resident on an SM.
-    const size_t smem = std::max<size_t>(Smem(n_max, several, ksplit).total, ksplit > 1 ? 77 * 1024 : 0);
+    // CTAs wait with their tensor memory allocated (for the grid before, for the cluster's others), so
+    // never more of them than it serves, two, may be on an SM (tc05.cuh).
+    const size_t smem = std::max<size_t>(Smem(n_max, several, ksplit).total, kShared);
     static bool configured[64] = {false};
     int dev = 0;
     cudaGetDevice(&dev);

@@ -82,7 +82,6 @@ sum_pflows_lanes_kernel(const float* __restrict__ nf, const float* __restrict__ 
                         int64_t ld, int B, const float* __restrict__ params, float* __restrict__ pf,
                         const PcbPflowTile* __restrict__ tiles, int rpb_log2, const int* __restrict__ cids,
                         const int* __restrict__ pids, const int* __restrict__ pfids, int32_t* __restrict__ status) {
-    pcb::pdl_trigger();
     using P = Plan<TKC>;
     constexpr int CP = TKC / 4;  // children per warp part
     extern __shared__ __align__(1024) uint8_t sm[];
@@ -103,7 +102,9 @@ sum_pflows_lanes_kernel(const float* __restrict__ nf, const float* __restrict__ 
         sPfid[i] = __ldg(pfids + k);
     }
     if (warp == 0) {
+        pcb::pdl_wait();
         tmem_alloc(slot, kCols);
+        pcb::pdl_trigger();  // not before: tc05.cuh
         fence_before_sync();
     }
     if (tid == 32) {

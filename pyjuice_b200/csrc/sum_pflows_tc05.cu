@@ -98,6 +98,7 @@ sum_pflows_tc05_kernel(const float* __restrict__ nf, const float* __restrict__ n
         sPfid[tid] = in ? __ldg(pfids + t.k_off + tid) : 0;
     }
     if (warp == 0) {
+        pcb::pdl_wait();
         tmem_alloc(slot, TKC);
         fence_before_sync();
     }
@@ -349,6 +350,7 @@ int launch(int cs, const float* nf, const float* nm, const float* em, int64_t ld
     const int slice = (int)pcb::cdiv(pcb::cdiv(B, cs), KB) * KB;
     using P = Plan<TKC, MODIFIED>;
     constexpr size_t smem = P::bytes();
+    static_assert(smem >= 102 * 1024, "clusters that share an SM must fit in its tensor memory (tc05.cuh)");
     static_assert(smem <= 227 * 1024, "shared memory");
     static bool configured[64] = {false};
     int dev = 0;

@@ -83,6 +83,21 @@ __device__ __forceinline__ float ex2(float x) {
     return y;
 }
 
+// An allocation waits, without a limit, until the SM has so many of its 512 columns free. So no CTA
+// that holds columns may wait for one that could be kept from allocating:
+// * A CTA that is started early must not hold columns that a CTA of the grid before it still
+//   wants. So the kernels allocate after their wait for that grid (pdl_wait), all but
+//   lse_tmem_kernel, whose launches lose 1 to 2 us by it when two of its CTAs start on an SM. It has 256
+//   columns and at least 77 KB of shared memory, of which an SM has 228 (a CTA takes 1 KB more than
+//   it asks for): two beside nothing else that allocates, or one beside one of lse_tc05.cu's kernels
+//   (at least 80 KB, up to 128 columns) or of sum_pflows_tc05.cu's (102 KB, up to 128). The persistent
+//   form (512 columns) asks for 152 KB, so never beside it; sum_pflows_lanes_kernel (up to 256 columns,
+//   two beside it) lets its successor start only after it has allocated.
+// * The CTAs of a cluster wait for one another with their columns held: those of lse_tmem_kernel
+//   and sum_pflows_tc05_kernel, which fit together as above.
+// (All early, with every successor held back behind the allocation: 0.5 to 2 us a launch. Shared
+// memory that keeps any CTAs of more than 512 columns apart: takes the L1 that the parameter flows
+// need, 291 -> 331 us for 200 regions of 256 x 256.)
 __device__ __forceinline__ void tmem_alloc(uint32_t* slot, uint32_t ncols) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(slot)),
                  "r"(ncols)
