@@ -53,9 +53,10 @@ class Autotuner:
         first eager call). ``run`` must launch on the current stream and overwrite its
         outputs, or write them to scratch."""
         k = self._key(key)
-        if k in self.choices:
-            if self.choices[k] in candidates:
-                return self.choices[k]
+        choice = self.choices.get(k)
+        if choice is not None:
+            if choice in candidates:
+                return choice
             # Kept by a call that had other forms on offer (alignment, settings): this set of them
             # has a choice of its own.
             k = self._key((k, "among") + tuple(candidates))

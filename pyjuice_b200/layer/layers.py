@@ -1033,8 +1033,9 @@ class SumLayer(Layer):
         d = self._desc(node_mars.device)
         B = node_mars.size(1)
         ld = node_mars.stride(0)
+        strides = (ld, 1)
         for t in (node_flows, element_flows, element_mars):
-            if t.stride(0) != ld or t.stride(1) != 1:
+            if t.stride() != strides:
                 raise ValueError("node/element mars/flows must share a row-major layout")
             if t.size(1) < B:  # the kernels would read or write past its last row
                 raise ValueError("node/element mars/flows must have a column for every sample")
