@@ -6,37 +6,34 @@
 
 namespace {
 
-// Sample of value q of thread position t: 4 consecutive samples per thread when rows allow
-// 16-byte accesses, else 4 samples 32 apart, so that a warp still reads and writes whole
-// 128-byte lines of rows whose start is not 16-byte aligned.
-template <bool VEC>
-__device__ __forceinline__ int sample_of(int t, int q) {
-    return VEC ? 4 * t + q : ((t >> 5) << 7) + 32 * q + (t & 31);
+// A thread takes 4 consecutive samples of a row, B of which are ngrp = ceil(B / 4) positions. (Rows
+// that do not allow 16-byte accesses: 4 scalar ones, whose lines the L1 keeps; 4 samples 32 or ngrp
+// apart are slower, 51200 rows of 2 x 65 samples: 14.4 us against 10.8.)
+//
+// Row (or group of rows) and position of this thread: positions run on from row to row, so that a
+// batch of any size leaves no lanes idle. 32-bit division where the numbers allow it.
+struct Place {
+    int64_t row;
+    int t;
+};
+__device__ __forceinline__ Place place_of(int ngrp, bool narrow) {
+    const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+    if (narrow) {
+        const uint32_t r = (uint32_t)i / (uint32_t)ngrp;
+        return {(int64_t)r, (int)((uint32_t)i - r * (uint32_t)ngrp)};
+    }
+    return {(int64_t)(i / (uint64_t)ngrp), (int)(i % (uint64_t)ngrp)};
 }
 
 template <bool VEC>
 __device__ __forceinline__ float4 load_row(const float* __restrict__ base, int64_t row, int64_t ld, int t, int B,
                                            float fill) {
-    if (VEC) return pcb::load4(base, row, ld, 4 * t, B, true, fill);
-    const float* p = base + row * ld;
-    float4 v;
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        const int b = sample_of<false>(t, q);
-        pcb::set(v, q, b < B ? __ldg(p + b) : fill);
-    }
-    return v;
+    return pcb::load4(base, row, ld, 4 * t, B, VEC, fill);
 }
 
 template <bool VEC>
 __device__ __forceinline__ void store_row(float* __restrict__ base, int64_t row, int64_t ld, int t, int B, float4 v) {
-    if (VEC) return pcb::store4(base, row, ld, 4 * t, B, true, v);
-    float* p = base + row * ld;
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        const int b = sample_of<false>(t, q);
-        if (b < B) p[b] = pcb::get(v, q);
-    }
+    pcb::store4(base, row, ld, 4 * t, B, VEC, v);
 }
 
 // Bound by HBM: arity reads and one write per output. A thread takes R consecutive rows of
@@ -51,15 +48,14 @@ template <int R, int J, bool VEC, bool ACCUM, bool LSE, bool MOD>
 __global__ void __launch_bounds__(256)
 prod_kernel(const float* __restrict__ in, float* __restrict__ out, int64_t ld, int B, const int* __restrict__ blk_row,
             const int* __restrict__ blk_off, const int* __restrict__ blk_cnt, const int* __restrict__ chs,
-            int blk_size, int ngrp, int num_chunks, int chunks_per_blk, int ctas_per_row, const float* __restrict__ nm,
+            int blk_size, int ngrp, int num_chunks, int chunks_per_blk, bool narrow, const float* __restrict__ nm,
             const int* __restrict__ mod_blk) {
     // The block tables (and the first J child indices) are read before the wait for the
     // previous kernel: they are compiled once and never written by a pass.
     pcb::pdl_trigger();
-    const int cta = (int)blockIdx.x / ctas_per_row;
-    const int chunk = cta * blockDim.y + threadIdx.y;
-    const int t = ((int)blockIdx.x - cta * ctas_per_row) * blockDim.x + threadIdx.x;
-    if (chunk >= num_chunks || t >= ngrp) return;
+    const Place at = place_of(ngrp, narrow);
+    if (at.row >= num_chunks) return;
+    const int chunk = (int)at.row, t = at.t;
     const int g = chunk / chunks_per_blk;
     const int i0 = (chunk - g * chunks_per_blk) * R;
     const int nr = R == 1 ? 1 : min(R, blk_size - i0);
@@ -153,22 +149,18 @@ int launch_prod(const char* name, const float* in, float* out, int64_t ld, int32
                 const int32_t* blk_off, const int32_t* blk_cnt, const int32_t* chs, int32_t num_blocks,
                 int32_t blk_size, const float* nm, const int32_t* mod_blk, void* stream) {
     const bool vec = pcb::vec_ok(in, ld) && pcb::vec_ok(out, ld) && (!MOD || pcb::vec_ok(nm, ld));
-    const int ngrp = (int)(vec ? pcb::cdiv(B, 4) : 32 * pcb::cdiv(B, 128));
+    const int ngrp = (int)pcb::cdiv(B, 4);
     // Four rows per thread once that still leaves two full sets of threads per SM.
     const bool wide = !LSE && blk_size >= 4 && (int64_t)num_blocks * blk_size / 4 * ngrp >= 2LL * pcb::num_sms() * 2048;
     const int rows = wide ? 4 : 1;
     const int per_blk = (int)pcb::cdiv(blk_size, rows);
     const int64_t chunks = (int64_t)num_blocks * per_blk;
-    int tx = 32;
-    while (tx < 256 && tx < ngrp) tx *= 2;
-    const int ty = 256 / tx;
-    const int64_t gx = pcb::cdiv(chunks, ty), gy = pcb::cdiv(ngrp, tx);
-    if (chunks > INT32_MAX - 1024 || gx * gy > INT32_MAX)
-        return pcb::set_error(PCB_E_ARG, "%s: layer or batch too large", name);
+    const int64_t ctas = pcb::cdiv(chunks * ngrp, 256);
+    if (chunks > INT32_MAX || ctas > INT32_MAX) return pcb::set_error(PCB_E_ARG, "%s: layer or batch too large", name);
     auto go = [&](auto kernel) {
-        return pcb::launch_status(pcb::launch_k(kernel, dim3((unsigned)(gx * gy)), dim3(tx, ty), 0,
-                                                pcb::as_stream(stream), 1u, in, out, ld, B, blk_row, blk_off, blk_cnt,
-                                                chs, blk_size, ngrp, (int)chunks, per_blk, (int)gy, nm, mod_blk), name);
+        return pcb::launch_status(pcb::launch_k(kernel, dim3((unsigned)ctas), dim3(256), 0, pcb::as_stream(stream), 1u,
+                                                in, out, ld, B, blk_row, blk_off, blk_cnt, chs, blk_size, ngrp,
+                                                (int)chunks, per_blk, ctas * 256 <= UINT32_MAX, nm, mod_blk), name);
     };
     if (wide) {
         if constexpr (!LSE)
@@ -177,37 +169,40 @@ int launch_prod(const char* name, const float* in, float* out, int64_t ld, int32
     return vec ? go(prod_kernel<1, 8, true, ACCUM, LSE, MOD>) : go(prod_kernel<1, 8, false, ACCUM, LSE, MOD>);
 }
 
-// out = log f - log m (out may be the flows themselves). Bound by HBM: four 16-byte (or four
-// times four strided 4-byte) accesses of each array in flight per thread. 51200 rows of 512
-// samples: 49 us (6.4 TB/s).
+// out = log f - log m (out may be the flows themselves). Bound by HBM: ROWS 16-byte accesses of each
+// array in flight per thread. Four rows where that leaves three quarters of the threads an SM holds
+// (51200 rows of 512 samples: 49 us, 6.4 TB/s; 16384 of 256: 7.7 us, 8.3 with one); one below, and where rows take scalar accesses, since four rows'
+// logarithms in one thread are a chain of 1 us (64 rows of 64 samples: 2.7 us against 1.6; 16384 of
+// 64: 4.7 against 3.1; 51200 of 209: 20.9 against 20.3).
 constexpr int kModRows = 4;
 
-template <bool VEC>
+template <int ROWS, bool VEC>
 __global__ void __launch_bounds__(256)
 modify_flows_kernel(const float* nf, const float* __restrict__ nm, float* out, int64_t ld, int B, int64_t row0,
-                    int64_t out_row0, int64_t num_rows, int ngrp, int ctas_per_row) {
-    pcb::pdl_begin();
-    const int64_t cta = (int64_t)blockIdx.x / ctas_per_row;
-    const int t = (int)((int64_t)blockIdx.x - cta * ctas_per_row) * blockDim.x + threadIdx.x;
-    if (t >= ngrp) return;
-    const int64_t r0 = (cta * blockDim.y + threadIdx.y) * kModRows;
-    float4 f[kModRows], m[kModRows];
+                    int64_t out_row0, int64_t num_rows, int ngrp, bool narrow) {
+    pcb::pdl_trigger();
+    const Place at = place_of(ngrp, narrow);
+    const int64_t r0 = at.row * ROWS;
+    const int t = at.t;
+    if (r0 >= num_rows) return;
+    pcb::pdl_wait();
+    float4 f[ROWS], m[ROWS];
 #pragma unroll
-    for (int r = 0; r < kModRows; ++r) {
+    for (int r = 0; r < ROWS; ++r) {
         if (r0 + r >= num_rows) break;
         if (VEC && 4 * t + 3 < B) {  // not the read-only path: out may be nf
             f[r] = *reinterpret_cast<const float4*>(nf + (row0 + r0 + r) * ld + 4 * t);
         } else {
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
-                const int b = sample_of<VEC>(t, q);
+                const int b = 4 * t + q;
                 pcb::set(f[r], q, b < B ? nf[(row0 + r0 + r) * ld + b] : 0.f);
             }
         }
         m[r] = load_row<VEC>(nm, row0 + r0 + r, ld, t, B, 0.f);
     }
 #pragma unroll
-    for (int r = 0; r < kModRows; ++r) {
+    for (int r = 0; r < ROWS; ++r) {
         if (r0 + r >= num_rows) break;
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
@@ -222,17 +217,17 @@ int launch_modify(const char* name, const float* nf, const float* nm, float* out
                   int64_t row1, int64_t out_row0, void* stream) {
     if (row1 == row0) return PCB_OK;
     const bool vec = pcb::vec_ok(nf, ld) && pcb::vec_ok(nm, ld) && pcb::vec_ok(out, ld);
-    const int ngrp = (int)(vec ? pcb::cdiv(B, 4) : 32 * pcb::cdiv(B, 128));
-    int tx = 32;
-    while (tx < 256 && tx < ngrp) tx *= 2;
-    const int64_t gy = pcb::cdiv(ngrp, tx), gx = pcb::cdiv(row1 - row0, (int64_t)kModRows * (256 / tx));
-    if (gx * gy > INT32_MAX) return pcb::set_error(PCB_E_ARG, "%s: too many rows", name);
+    const int ngrp = (int)pcb::cdiv(B, 4);
+    const bool wide = vec && (row1 - row0) / kModRows * ngrp >= pcb::num_sms() * 1536LL;
+    const int64_t ctas = pcb::cdiv(pcb::cdiv(row1 - row0, wide ? kModRows : 1) * ngrp, 256);
+    if (ctas > INT32_MAX) return pcb::set_error(PCB_E_ARG, "%s: too many rows", name);
     auto go = [&](auto kernel) {
-        return pcb::launch_status(pcb::launch_k(kernel, dim3((unsigned)(gx * gy)), dim3(tx, 256 / tx), 0,
-                                                pcb::as_stream(stream), 1u, nf, nm, out, ld, B, row0, out_row0,
-                                                row1 - row0, ngrp, (int)gy), name);
+        return pcb::launch_status(pcb::launch_k(kernel, dim3((unsigned)ctas), dim3(256), 0, pcb::as_stream(stream), 1u,
+                                                nf, nm, out, ld, B, row0, out_row0, row1 - row0, ngrp,
+                                                ctas * 256 <= UINT32_MAX), name);
     };
-    return vec ? go(modify_flows_kernel<true>) : go(modify_flows_kernel<false>);
+    if (wide) return go(modify_flows_kernel<kModRows, true>);
+    return vec ? go(modify_flows_kernel<1, true>) : go(modify_flows_kernel<1, false>);
 }
 
 }  // namespace
