@@ -164,6 +164,14 @@ int pcb_input_cat_em(float* params, const float* param_flows, const int32_t* s_p
                      double step_size, double pseudocount, int32_t keep_zero_params, void* stream);
 
 /*
+ * pcb_input_cat_em with several nodes per warp, for many nodes of up to 256 categories (larger ones
+ * are taken too, more slowly). Same arguments; the same values but for the order of a node's sum.
+ */
+int pcb_input_cat_em_many(float* params, const float* param_flows, const int32_t* s_pids, const int32_t* s_pfids,
+                     const int32_t* ncats, const int32_t* source_nids, int32_t num_source_nodes,
+                     double step_size, double pseudocount, int32_t keep_zero_params, void* stream);
+
+/*
  * Bernoulli (kind 1), Gaussian (kind 2) and DiscreteLogistic (kind 3) input layers; data is
  * FP32 [num_vars, data_ld] (Bernoulli reads x > 0; DiscreteLogistic reads bin indices),
  * missing values indexed as in pcb_input_cat_fwd. meta: per-node metadata indexed by the
@@ -638,6 +646,10 @@ int pcb_sum_em_f64flows(float* params, const double* param_flows, const int64_t*
                         const int32_t* blk_nch, const int32_t* blk_bs, int32_t num_blocks, double step_size,
                         double pseudocount, int32_t keep_zero_params, void* stream);
 int pcb_input_cat_em_f64flows(float* params, const double* param_flows, const int32_t* s_pids,
+                              const int32_t* s_pfids, const int32_t* ncats, const int32_t* source_nids,
+                              int32_t num_source_nodes, double step_size, double pseudocount,
+                              int32_t keep_zero_params, void* stream);
+int pcb_input_cat_em_many_f64flows(float* params, const double* param_flows, const int32_t* s_pids,
                               const int32_t* s_pfids, const int32_t* ncats, const int32_t* source_nids,
                               int32_t num_source_nodes, double step_size, double pseudocount,
                               int32_t keep_zero_params, void* stream);

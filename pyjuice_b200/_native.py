@@ -100,6 +100,8 @@ _SIGS = {
                            c_void_p, c_void_p, c_int32, c_void_p], c_int32),
     "pcb_input_cat_em": ([c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int32, c_double, c_double,
                           c_int32, c_void_p], c_int32),
+    "pcb_input_cat_em_many": ([c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int32, c_double, c_double,
+                          c_int32, c_void_p], c_int32),
     "pcb_input_dist_fwd": ([c_int32, c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_void_p, c_int32, c_int32,
                             c_void_p, c_int64, c_int32, c_void_p, c_int64, c_int64, c_void_p], c_int32),
     "pcb_input_dist_bwd": ([c_int32, c_void_p, c_int64, c_void_p, c_int64, c_int32, c_void_p, c_void_p, c_void_p,
@@ -165,6 +167,8 @@ _SIGS = {
     "pcb_sum_em_f64flows": ([c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int32, c_double,
                              c_double, c_int32, c_void_p], c_int32),
     "pcb_input_cat_em_f64flows": ([c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int32, c_double,
+                                   c_double, c_int32, c_void_p], c_int32),
+    "pcb_input_cat_em_many_f64flows": ([c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int32, c_double,
                                    c_double, c_int32, c_void_p], c_int32),
     "pcb_flows_accumulate_f64": ([c_void_p, c_void_p, c_int64, c_void_p], c_int32),
     "pcb_pflow_accum_f64": ([c_void_p, c_int64, c_int64, c_void_p, c_int32, c_void_p], c_int32),

@@ -109,13 +109,75 @@ sum_em_kernel(float* __restrict__ params, const FT* __restrict__ pflows, const i
     }
 }
 
-// Input EM, bound by HBM (flows and parameters read, parameters written). A warp takes
+// (p, f, inv = step / sum) -> new parameter; one FP64 reciprocal per node: the sum holds the
+// pseudocounts in the keep-zero form, else pc is added to it
+template <bool KEEP_ZERO>
+__device__ __forceinline__ float em_update(double p, double f, double pcn, double step, double inv) {
+    if (KEEP_ZERO && p < 1e-12) return 0.f;
+    return (float)((1.0 - step) * p + (f + pcn) * inv);
+}
+
+// The flow that a category adds to its node's sum
+template <bool KEEP_ZERO, typename FT>
+__device__ __forceinline__ double em_term(float p, FT f, double pcn) {
+    if (KEEP_ZERO) return p < 1e-12f ? 0.0 : (double)f + pcn;
+    return (double)f;
+}
+
+// Input EM of one node by one warp, categories strided over the lanes, any number of categories:
+// up to 256 in registers (all loads at once, one pass over memory), more in two passes.
+template <bool KEEP_ZERO, typename FT>
+__device__ __forceinline__ void em_node(float* __restrict__ params, const FT* __restrict__ pflows, int64_t sp,
+                                        int64_t sf, int K, int lane, double step, double pc) {
+    constexpr int R = 8;
+    const double pcn = pc / (double)K;
+    double s = 0.0;
+    if (K <= 32 * R) {
+        FT f[R];
+        float p[R];
+#pragma unroll
+        for (int j = 0; j < R; ++j) {
+            const int k = lane + 32 * j;
+            f[j] = k < K ? pflows[sf + k] : FT(0);
+            p[j] = k < K ? params[sp + k] : 0.f;
+        }
+#pragma unroll
+        for (int j = 0; j < R; ++j)
+            if (lane + 32 * j < K) s += em_term<KEEP_ZERO>(p[j], f[j], pcn);
+        s = pcb::warp_sum(s);
+        const double inv = KEEP_ZERO ? step / s : step / (s + pc);
+#pragma unroll
+        for (int j = 0; j < R; ++j) {
+            const int k = lane + 32 * j;
+            if (k < K) params[sp + k] = em_update<KEEP_ZERO>((double)p[j], (double)f[j], pcn, step, inv);
+        }
+        return;
+    }
+    for (int k = lane; k < K; k += 32) s += em_term<KEEP_ZERO>(KEEP_ZERO ? params[sp + k] : 0.f, pflows[sf + k], pcn);
+    s = pcb::warp_sum(s);
+    const double inv = KEEP_ZERO ? step / s : step / (s + pc);
+    for (int k = lane; k < K; k += 32)
+        params[sp + k] = em_update<KEEP_ZERO>((double)params[sp + k], (double)pflows[sf + k], pcn, step, inv);
+}
+
+template <bool KEEP_ZERO, typename FT>
+__global__ void __launch_bounds__(256)
+input_em_node_kernel(float* __restrict__ params, const FT* __restrict__ pflows, const int* __restrict__ s_pids,
+                     const int* __restrict__ s_pfids, const int* __restrict__ ncats,
+                     const int* __restrict__ source_nids, int num_src, double step, double pc) {
+    pcb::pdl_wait();  // no early trigger, as in sum_em_kernel
+    const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (w >= num_src) return;
+    const int n = source_nids[w];
+    em_node<KEEP_ZERO>(params, pflows, (int64_t)s_pids[n], (int64_t)s_pfids[n], ncats[n], threadIdx.x & 31, step, pc);
+}
+
+// The same for many nodes, bound by HBM (flows and parameters read, parameters written). A warp takes
 // nodes_per_warp consecutive source nodes. Nodes of up to 256 categories go 32 / G at a time,
 // G = 8, 16 or 32 lanes to a node and up to 8 categories to a lane (two 16-byte accesses where
 // the slabs are aligned), and the next nodes' values are loaded before the current ones are
 // summed, so that no warp waits on one node's chain of table and value loads. 200704 nodes of
-// 64 categories: 37 us (4.2 TB/s), against 281 us with one node per warp; larger nodes take
-// two passes over memory.
+// 64 categories: 37 us (4.2 TB/s), against 281 us with one node per warp.
 constexpr int kEmNodes = 16;  // most nodes per warp
 
 template <bool KEEP_ZERO, typename FT>
@@ -136,14 +198,6 @@ input_em_kernel(float* __restrict__ params, const FT* __restrict__ pflows, const
     }
     pcb::pdl_wait();  // no early trigger, as in sum_em_kernel
     if (cnt <= 0) return;
-    // one FP64 reciprocal per node: inv = step / s (keep-zero form) or step / (s + pc)
-    auto scale = [&](double s) -> double { return KEEP_ZERO ? step / s : step / (s + pc); };
-    auto update = [&](double p, double f, double inv, double pcn) -> float {
-        double np;
-        if (KEEP_ZERO) np = (p < 1e-12) ? 0.0 : (1.0 - step) * p + (f + pcn) * inv;
-        else np = (1.0 - step) * p + (f + pcn) * inv;
-        return (float)np;
-    };
     const int maxK = __reduce_max_sync(0xffffffffu, myK);
     if (maxK <= 256) {
         const int G = maxK <= 64 ? 8 : (maxK <= 128 ? 16 : 32);
@@ -199,18 +253,18 @@ input_em_kernel(float* __restrict__ params, const FT* __restrict__ pflows, const
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
                 if (4 * gl + 4 * G * (j >> 2) + (j & 3) >= cur.K) continue;
-                if (KEEP_ZERO) s += (cur.p[j] < 1e-12f) ? 0.0 : (double)cur.f[j] + pcn;
-                else s += (double)cur.f[j];
+                s += em_term<KEEP_ZERO>(cur.p[j], cur.f[j], pcn);
             }
             for (int o = G >> 1; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-            const double inv = scale(s);
+            const double inv = KEEP_ZERO ? step / s : step / (s + pc);
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 const int k = 4 * gl + 4 * G * h;
                 float4 o;
 #pragma unroll
                 for (int q = 0; q < 4; ++q)
-                    pcb::set(o, q, update((double)cur.p[4 * h + q], (double)cur.f[4 * h + q], inv, pcn));
+                    pcb::set(o, q, em_update<KEEP_ZERO>((double)cur.p[4 * h + q], (double)cur.f[4 * h + q], pcn, step,
+                                                        inv));
                 if (aligned) {
                     if (k < cur.K) *reinterpret_cast<float4*>(params + cur.sp + k) = o;
                 } else {
@@ -223,22 +277,9 @@ input_em_kernel(float* __restrict__ params, const FT* __restrict__ pflows, const
         }
         return;
     }
-    for (int i = 0; i < cnt; ++i) {
-        const int K = __shfl_sync(0xffffffffu, myK, i);
-        const int64_t sp = __shfl_sync(0xffffffffu, mySp, i);
-        const int64_t sf = __shfl_sync(0xffffffffu, mySf, i);
-        const double pcn = pc / (double)K;
-        double s = 0.0;
-        for (int k = lane; k < K; k += 32) {
-            const double f = (double)pflows[sf + k];
-            if (KEEP_ZERO) s += (params[sp + k] < 1e-12f) ? 0.0 : f + pcn;
-            else s += f;
-        }
-        s = pcb::warp_sum(s);
-        const double inv = scale(s);
-        for (int k = lane; k < K; k += 32)
-            params[sp + k] = update((double)params[sp + k], (double)pflows[sf + k], inv, pcn);
-    }
+    for (int i = 0; i < cnt; ++i)
+        em_node<KEEP_ZERO>(params, pflows, (int64_t)__shfl_sync(0xffffffffu, mySp, i),
+                           (int64_t)__shfl_sync(0xffffffffu, mySf, i), __shfl_sync(0xffffffffu, myK, i), lane, step, pc);
 }
 
 template <typename FT>
@@ -263,23 +304,25 @@ int sum_em_launch(float* params, const FT* param_flows, const int64_t* blk_pbase
 template <typename FT>
 int input_em_launch(float* params, const FT* param_flows, const int32_t* s_pids, const int32_t* s_pfids,
                     const int32_t* ncats, const int32_t* source_nids, int32_t num_source_nodes, double step_size,
-                    double pseudocount, int32_t keep_zero_params, void* stream, const char* name) {
+                    double pseudocount, int32_t keep_zero_params, void* stream, const char* name, bool many) {
     if (!params || !param_flows || !s_pids || !s_pfids || !ncats || !source_nids || num_source_nodes < 0)
         return pcb::set_error(PCB_E_ARG, "%s: bad arguments", name);
     if (!(step_size > 0.0 && step_size <= 1.0)) return pcb::set_error(PCB_E_ARG, "%s: step_size must be in (0, 1]", name);
     if (num_source_nodes == 0) return PCB_OK;
-    // several nodes per warp only once that leaves 16 warps per SM
-    const int npw = (int)std::max<int64_t>(1, std::min<int64_t>(kEmNodes, num_source_nodes / (pcb::num_sms() * 16)));
-    const unsigned grid = (unsigned)pcb::cdiv(pcb::cdiv(num_source_nodes, npw) * 32, 256);
     cudaStream_t s = pcb::as_stream(stream);
-    if (keep_zero_params) {
-        return pcb::launch_status(pcb::launch_k(input_em_kernel<true, FT>, dim3(grid), dim3(256), 0, s, 1u, params,
-                                                param_flows, s_pids, s_pfids, ncats, source_nids, num_source_nodes,
-                                                npw, step_size, pseudocount), name);
+    if (!many) {
+        const dim3 grid((unsigned)pcb::cdiv((int64_t)num_source_nodes * 32, 256));
+        return pcb::launch_status(
+            pcb::launch_k(keep_zero_params ? input_em_node_kernel<true, FT> : input_em_node_kernel<false, FT>, grid,
+                          dim3(256), 0, s, 1u, params, param_flows, s_pids, s_pfids, ncats, source_nids,
+                          num_source_nodes, step_size, pseudocount), name);
     }
-    return pcb::launch_status(pcb::launch_k(input_em_kernel<false, FT>, dim3(grid), dim3(256), 0, s, 1u, params,
-                                            param_flows, s_pids, s_pfids, ncats, source_nids, num_source_nodes,
-                                            npw, step_size, pseudocount), name);
+    const int npw = (int)std::max<int64_t>(1, std::min<int64_t>(kEmNodes, num_source_nodes / (pcb::num_sms() * 16)));
+    const dim3 grid((unsigned)pcb::cdiv(pcb::cdiv(num_source_nodes, npw) * 32, 256));
+    return pcb::launch_status(
+        pcb::launch_k(keep_zero_params ? input_em_kernel<true, FT> : input_em_kernel<false, FT>, grid, dim3(256), 0, s,
+                      1u, params, param_flows, s_pids, s_pfids, ncats, source_nids, num_source_nodes, npw, step_size,
+                      pseudocount), name);
 }
 
 // acc[i] += flows[i]: 4 elements per thread, grid-stride.
@@ -425,7 +468,14 @@ extern "C" int pcb_input_cat_em(float* params, const float* param_flows, const i
                                 const int32_t* ncats, const int32_t* source_nids, int32_t num_source_nodes,
                                 double step_size, double pseudocount, int32_t keep_zero_params, void* stream) {
     return input_em_launch<float>(params, param_flows, s_pids, s_pfids, ncats, source_nids, num_source_nodes,
-                                  step_size, pseudocount, keep_zero_params, stream, "pcb_input_cat_em");
+                                  step_size, pseudocount, keep_zero_params, stream, "pcb_input_cat_em", false);
+}
+
+extern "C" int pcb_input_cat_em_many(float* params, const float* param_flows, const int32_t* s_pids, const int32_t* s_pfids,
+                                const int32_t* ncats, const int32_t* source_nids, int32_t num_source_nodes,
+                                double step_size, double pseudocount, int32_t keep_zero_params, void* stream) {
+    return input_em_launch<float>(params, param_flows, s_pids, s_pfids, ncats, source_nids, num_source_nodes,
+                                  step_size, pseudocount, keep_zero_params, stream, "pcb_input_cat_em_many", true);
 }
 
 extern "C" int pcb_input_cat_em_f64flows(float* params, const double* param_flows, const int32_t* s_pids,
@@ -433,7 +483,15 @@ extern "C" int pcb_input_cat_em_f64flows(float* params, const double* param_flow
                                          int32_t num_source_nodes, double step_size, double pseudocount,
                                          int32_t keep_zero_params, void* stream) {
     return input_em_launch<double>(params, param_flows, s_pids, s_pfids, ncats, source_nids, num_source_nodes,
-                                   step_size, pseudocount, keep_zero_params, stream, "pcb_input_cat_em_f64flows");
+                                   step_size, pseudocount, keep_zero_params, stream, "pcb_input_cat_em_f64flows", false);
+}
+
+extern "C" int pcb_input_cat_em_many_f64flows(float* params, const double* param_flows, const int32_t* s_pids,
+                                         const int32_t* s_pfids, const int32_t* ncats, const int32_t* source_nids,
+                                         int32_t num_source_nodes, double step_size, double pseudocount,
+                                         int32_t keep_zero_params, void* stream) {
+    return input_em_launch<double>(params, param_flows, s_pids, s_pfids, ncats, source_nids, num_source_nodes,
+                                   step_size, pseudocount, keep_zero_params, stream, "pcb_input_cat_em_many_f64flows", true);
 }
 
 extern "C" int pcb_flows_accumulate_f64(double* acc, const float* flows, int64_t n, void* stream) {

@@ -1709,6 +1709,14 @@ class InputLayer(Layer, torch.nn.Module):
         if self.kind == 4 and "categorical_evidence_logp_grad" in kwargs:
             self._backward_poe_evidence(data, node_flows, node_mars, d, B, logspace_flows, kwargs)
 
+    @staticmethod
+    def _em_many(num_nodes: int, max_ncats: int) -> bool:
+        """Whether the EM update takes several nodes per warp (pcb_input_cat_em_many). Measured (us, one
+        node per warp / several): 12,544 nodes of 64 categories 6.8 / 6.4, 20,000: 9.4 / 6.2, 200,704: 104 /
+        37; 32,768 of 256: 16.1 / 24.6, 49,152: 38.2 / 36.3, 200,704: 153 / 120; 4,096 of 2: 3.6 / 5.0; 65,536 of
+        300: 86 / 179; 4,096 of 5,000: 62 / 161."""
+        return num_nodes >= 16384 if max_ncats <= 64 else max_ncats <= 256 and num_nodes >= 49152
+
     def mini_batch_em(self, step_size: float, pseudocount: float = 0.0, keep_zero_params: bool = False,
                       use_f64_flows: bool = False):
         d = self._desc(self.params.device)
@@ -1725,8 +1733,9 @@ class InputLayer(Layer, torch.nn.Module):
                      nat.ptr(d["s_pfids"]), nat.ptr(d["node_meta"]), nat.ptr(d["source_nids"]),
                      d["source_nids"].size(0), float(step_size), float(pseudocount), nat.stream())
             return
-        nat.call("pcb_input_cat_em_f64flows" if use_f64_flows else "pcb_input_cat_em", nat.ptr(self.params),
-                 nat.ptr(pf), nat.ptr(d["s_pids"]), nat.ptr(d["s_pfids"]), nat.ptr(d["ncats"]),
+        many = "_many" if self._em_many(d["source_nids"].size(0), d["max_ncats"]) else ""
+        nat.call(f"pcb_input_cat_em{many}" + ("_f64flows" if use_f64_flows else ""), nat.ptr(self.params), nat.ptr(pf),
+                 nat.ptr(d["s_pids"]), nat.ptr(d["s_pfids"]), nat.ptr(d["ncats"]),
                  nat.ptr(d["source_nids"]), d["source_nids"].size(0), float(step_size), float(pseudocount),
                  1 if keep_zero_params else 0, nat.stream())
 

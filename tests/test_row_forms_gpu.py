@@ -30,3 +30,43 @@ def test_flow_ratios(rows, B, cuda_device):
         # logf within 1 ulp of a magnitude up to 17, the difference rounded once
         assert torch.all((got.double() - want)[fin].abs() <= 2.0 ** -19 + 2.0 ** -24 * want[fin].abs())
     assert torch.all(out[rows] == 7.0) and torch.equal(flows[0], nf[0])
+
+
+def _input_layer(variables, nodes, bs, cats, device):
+    with juice.set_block_size(bs):
+        leaves = [juice.inputs(v, num_node_blocks=nodes // bs, dist=Categorical(num_cats=cats)) for v in range(variables)]
+    return juice.InputLayer(leaves, cum_nodes=bs, pc_num_vars=variables).to(device)
+
+
+@pytest.mark.parametrize("variables,nodes,bs,cats", [(1, 1, 1, 2), (7, 12, 4, 5), (3, 16, 16, 64), (5, 40, 8, 257),
+                                                     (300, 64, 32, 30), (2, 8, 8, 1000)])
+@pytest.mark.parametrize("keep_zero", [False, True])
+@pytest.mark.parametrize("f64", [False, True])
+def test_em_forms(variables, nodes, bs, cats, keep_zero, f64, cuda_device, monkeypatch):
+    """One node per warp and several: the same FP64 update, sums in another order."""
+    layer = _input_layer(variables, nodes, bs, cats, cuda_device)
+    gen = torch.Generator(device=cuda_device).manual_seed(cats + nodes)
+    theta = torch.rand(layer.params.shape, generator=gen, device=cuda_device) + 0.01
+    theta[torch.rand(theta.shape, generator=gen, device=cuda_device) < 0.2] = 0.0
+    flows = torch.rand([max(layer.num_param_flows, 1)], generator=gen, device=cuda_device)
+    got = []
+    for many in (False, True):
+        monkeypatch.setattr(type(layer), "_em_many", staticmethod(lambda n, k: many))
+        with torch.no_grad():
+            layer.params.copy_(theta)
+        layer.init_param_flows(0.0)
+        layer.param_flows.copy_(flows)
+        if f64:
+            layer.init_param_flows_f64()
+            layer.param_flows_f64.copy_(flows.double())
+        layer.mini_batch_em(step_size=0.3, pseudocount=0.1, keep_zero_params=keep_zero, use_f64_flows=f64)
+        got.append(layer.params.clone())
+    assert torch.isfinite(got[0]).all()
+    # sums of FP64 differ by a few 2^-53, so the rounded results by at most one unit in the last place
+    assert torch.all((got[0] - got[1]).abs() <= 2.0 ** -23 * got[0].abs())
+
+
+def test_em_rule():
+    layer = juice.InputLayer
+    assert [layer._em_many(n, k) for n, k in ((16383, 64), (16384, 64), (49151, 256), (49152, 256), (10 ** 6, 257))] == \
+        [False, True, False, True, False]
