@@ -131,6 +131,15 @@ int pcb_input_cat_fwd(const int64_t* data, int64_t data_ld, const float* params,
                       int64_t miss_sb, int64_t miss_sv, void* stream);
 
 /*
+ * pcb_input_cat_fwd for vocabularies of up to 256 categories (four nodes of a variable share a
+ * look-up; larger ones are taken too, more slowly). Same arguments and values.
+ */
+int pcb_input_cat_fwd_quads(const int64_t* data, int64_t data_ld, const float* params,
+                      const int32_t* vids, const int32_t* s_pids, const int32_t* ncats, int32_t num_nodes,
+                      int32_t node_offset, float* node_mars, int64_t ld, int32_t B, const uint8_t* missing,
+                      int64_t miss_sb, int64_t miss_sv, void* stream);
+
+/*
  * Categorical input layer backward (parameter flows), deterministic:
  * param_flows[s_pfids[n] + k] += sum_{b : data[v, b] == k} node_flows[node_offset + n, b]
  * for every node n of every variable group. Groups are runs of nodes over the same

@@ -95,6 +95,8 @@ _SIGS = {
                         c_void_p], c_int32),
     "pcb_input_cat_fwd": ([c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_void_p, c_int32, c_int32, c_void_p,
                            c_int64, c_int32, c_void_p, c_int64, c_int64, c_void_p], c_int32),
+    "pcb_input_cat_fwd_quads": ([c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_void_p, c_int32, c_int32, c_void_p,
+                                 c_int64, c_int32, c_void_p, c_int64, c_int64, c_void_p], c_int32),
     "pcb_input_cat_bwd": ([c_void_p, c_int64, c_void_p, c_int64, c_int32, c_void_p, c_void_p, c_void_p, c_void_p,
                            c_int32, c_int32, c_void_p, c_int32, c_void_p, c_int32, c_void_p, c_int64, c_int64,
                            c_void_p, c_void_p, c_int32, c_void_p], c_int32),

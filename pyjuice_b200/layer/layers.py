@@ -1539,8 +1539,8 @@ class InputLayer(Layer, torch.nn.Module):
         part = self._partial("fw", node_mars.device)
         runs = [(0, self.num_nodes)] if part is None else part["runs"]
         for n0, cnt in runs:  # the node tables are passed from the run's first node on
-            nat.call("pcb_input_cat_fwd", nat.ptr(data), data.stride(0), nat.ptr(self.params),
-                     c_void_p(d["vids"].data_ptr() + 4 * n0), c_void_p(d["s_pids"].data_ptr() + 4 * n0),
+            nat.call("pcb_input_cat_fwd_quads" if d["max_ncats"] <= 256 else "pcb_input_cat_fwd", nat.ptr(data),
+                     data.stride(0), nat.ptr(self.params), c_void_p(d["vids"].data_ptr() + 4 * n0), c_void_p(d["s_pids"].data_ptr() + 4 * n0),
                      c_void_p(d["ncats"].data_ptr() + 4 * n0), cnt, self._output_ind_range[0] + n0,
                      nat.ptr(node_mars), node_mars.stride(0), B, nat.ptr(m), sb, sv, nat.stream())
 

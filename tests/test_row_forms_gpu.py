@@ -70,3 +70,29 @@ def test_em_rule():
     layer = juice.InputLayer
     assert [layer._em_many(n, k) for n, k in ((16383, 64), (16384, 64), (49151, 256), (49152, 256), (10 ** 6, 257))] == \
         [False, True, False, True, False]
+
+
+# quads of one variable and not, categories in shared memory and not, ragged batches
+@pytest.mark.parametrize("variables,nodes,bs,cats,B", [(1, 1, 1, 2, 1), (5, 6, 2, 17, 33), (3, 16, 16, 256, 130), (4, 20, 4, 257, 515),
+                                                       (2, 32, 32, 3000, 64)])
+def test_value_forms(variables, nodes, bs, cats, B, cuda_device):
+    """Eight nodes per CTA and quads of nodes: the same logarithms, to the bit, with missing values and
+    categories that do not exist."""
+    nat.device_status()
+    layer = _input_layer(variables, nodes, bs, cats, cuda_device)
+    d = layer._desc(cuda_device)
+    gen = torch.Generator(device=cuda_device).manual_seed(cats + B)
+    with torch.no_grad():
+        layer.params.copy_(torch.rand(layer.params.shape, generator=gen, device=cuda_device) + 1e-4)
+    data = torch.randint(0, cats, [variables, B], generator=gen, device=cuda_device)
+    data[0, 0] = cats
+    mask = (torch.rand([B, variables], generator=gen, device=cuda_device) < 0.2).to(torch.uint8)
+    got = []
+    for name in ("pcb_input_cat_fwd", "pcb_input_cat_fwd_quads"):
+        nm = torch.full([bs + variables * nodes, B], 3.0, device=cuda_device)
+        nat.call(name, nat.ptr(data), B, nat.ptr(layer.params), nat.ptr(d["vids"]), nat.ptr(d["s_pids"]),
+                 nat.ptr(d["ncats"]), variables * nodes, bs, nat.ptr(nm), B, B, nat.ptr(mask), variables, 1, nat.stream())
+        got.append(nm)
+    assert torch.equal(got[0].nan_to_num(nan=9.0), got[1].nan_to_num(nan=9.0))
+    assert torch.all(got[0][:bs] == 3.0)
+    assert nat.device_status() == (0 if mask[0, 0] else 4)
