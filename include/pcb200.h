@@ -162,6 +162,17 @@ int pcb_input_cat_bwd(const int64_t* data, int64_t data_ld, const float* node_fl
                       const int32_t* s_pids, const float* params, int32_t atomic, void* stream);
 
 /*
+ * pcb_input_cat_bwd with one node per lane, for variables with many nodes (tiles of 32 nodes
+ * share one sort of the batch). Same arguments and sums; vocabularies of up to 8 million.
+ */
+int pcb_input_cat_bwd_tiles(const int64_t* data, int64_t data_ld, const float* node_flows, int64_t ld, int32_t B,
+                            const int32_t* grp_var, const int32_t* grp_node0, const int32_t* grp_count,
+                            const int32_t* grp_ncats, int32_t num_groups, int32_t max_ncats,
+                            const int32_t* s_pfids, int32_t node_offset, float* param_flows,
+                            int32_t logspace_flows, const uint8_t* missing, int64_t miss_sb, int64_t miss_sv,
+                            const int32_t* s_pids, const float* params, int32_t atomic, void* stream);
+
+/*
  * Categorical EM update of the source nodes (in FP64):
  *   theta' = (1 - s) * theta + s * (f + pc / K) / (sum_k f + pc)
  * (keep_zero_params: zero parameters stay zero and the normaliser excludes them).

@@ -1701,13 +1701,27 @@ class InputLayer(Layer, torch.nn.Module):
         g = self._partial("bk", node_flows.device) or d
         if g["grp_var"].numel() == 0:
             return
-        nat.call("pcb_input_cat_bwd", nat.ptr(data), data.stride(0), nat.ptr(node_flows), node_flows.stride(0), B,
+        nat.call("pcb_input_cat_bwd_tiles" if self._bwd_tiles(d["max_grp"], d["max_ncats"], d["grp_var"].size(0), B)
+                 else "pcb_input_cat_bwd", nat.ptr(data), data.stride(0), nat.ptr(node_flows), node_flows.stride(0), B,
                  nat.ptr(g["grp_var"]), nat.ptr(g["grp_node0"]), nat.ptr(g["grp_count"]), nat.ptr(g["grp_ncats"]),
                  g["grp_var"].size(0), d["max_ncats"], nat.ptr(d["s_pfids"]), self._output_ind_range[0],
                  nat.ptr(self.param_flows), 1 if logspace_flows else 0, nat.ptr(m), sb, sv, nat.ptr(d["s_pids"]),
                  nat.ptr(self.params), 1 if d["shared_slots"] else 0, nat.stream())
         if self.kind == 4 and "categorical_evidence_logp_grad" in kwargs:
             self._backward_poe_evidence(data, node_flows, node_mars, d, B, logspace_flows, kwargs)
+
+    @staticmethod
+    def _bwd_tiles(nodes: int, max_ncats: int, num_vars: int, B: int) -> bool:
+        """Whether the flow histogram takes 32 nodes of a variable side by side (pcb_input_cat_bwd_tiles):
+        from a full tile on; where the batch meets hundreds of categories of many variables, the slots'
+        updates dominate, which one node per warp spreads better. Measured (us, one node per warp / tiles):
+        784 variables of 32 nodes, 64 categories, batch 512: 37.7 / 31.7, of 128: 125 / 85.5, of 16, batch
+        1000: 42.7 / 54.7; 400 of 8, 10 categories, batch 129: 5.7 / 10.5; 784 of 64 nodes, 600 categories,
+        batch 129: 69.9 / 51.0, 512: 142 / 188, 1000: 218 / 325; 64 of 64, 2000 categories, batch 512: 67.4 /
+        18.3; 2000 of 32 nodes, 256 categories, batch 512: 102 / 113 (one sort of the batch per tile)."""
+        if nodes < 32 or (nodes < 64 and num_vars > 1024):
+            return False
+        return max_ncats <= 256 or B <= 256 or num_vars * nodes < 8 * 2048
 
     @staticmethod
     def _em_many(num_nodes: int, max_ncats: int) -> bool:

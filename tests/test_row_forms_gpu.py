@@ -96,3 +96,45 @@ def test_value_forms(variables, nodes, bs, cats, B, cuda_device):
     assert torch.equal(got[0].nan_to_num(nan=9.0), got[1].nan_to_num(nan=9.0))
     assert torch.all(got[0][:bs] == 3.0)
     assert nat.device_status() == (0 if mask[0, 0] else 4)
+
+
+@pytest.mark.parametrize("variables,nodes,bs,cats,B", [(1, 1, 1, 2, 1), (5, 6, 2, 17, 33), (3, 32, 16, 256, 130), (4, 33, 1, 300, 515),
+                                                       (2, 96, 32, 3000, 1100), (1, 4, 4, 45000, 1024)])
+@pytest.mark.parametrize("missing", [False, True])
+@pytest.mark.parametrize("log", [False, True])
+def test_histogram_forms(variables, nodes, bs, cats, B, missing, log, cuda_device, monkeypatch):
+    """One node per warp and one per lane: flows per category against FP64, vocabularies of more than
+    40,000 categories at a batch of 1024 on the second (the first refuses them)."""
+    layer = _input_layer(variables, nodes, bs, cats, cuda_device)
+    gen = torch.Generator(device=cuda_device).manual_seed(cats + B)
+    with torch.no_grad():
+        layer.params.copy_(torch.rand(layer.params.shape, generator=gen, device=cuda_device) / cats)
+    data = torch.randint(0, cats, [variables, B], generator=gen, device=cuda_device)
+    nf = torch.rand([bs + variables * nodes, B], generator=gen, device=cuda_device)
+    mask = torch.rand([B, variables], generator=gen, device=cuda_device) < 0.2 if missing else None
+    flows = nf.double()[bs:].reshape(variables, nodes, B)
+    want = torch.zeros([variables, nodes, cats], dtype=torch.float64, device=cuda_device)
+    seen = flows if mask is None else flows * (~mask).T[:, None, :]
+    want.scatter_add_(2, data[:, None, :].expand(variables, nodes, B), seen)
+    if mask is not None:
+        theta = layer.params.double().reshape(variables, nodes, cats)
+        want += (flows - seen).sum(dim=2, keepdim=True) * theta
+    for tiles in (False, True):
+        monkeypatch.setattr(type(layer), "_bwd_tiles", staticmethod(lambda *a: tiles))
+        layer.init_param_flows(0.0)
+        run = lambda: layer.backward(data, nf.log() if log else nf, nf, missing_mask=mask, logspace_flows=log)
+        if cats > 40000 and not tiles:
+            with pytest.raises(RuntimeError):
+                run()
+            continue
+        run()
+        got = layer.param_flows.double().reshape(want.shape)
+        # up to B additions rounded once each, the exponential's and logarithm's 2^-21
+        assert torch.all((got - want).abs() <= (B * 2.0 ** -24 + (2.0 ** -20 if log else 0.0)) * want + 1e-12)
+
+
+def test_histogram_rule():
+    tiles = juice.InputLayer._bwd_tiles  # nodes of a variable, categories, variables, batch
+    assert [tiles(*a) for a in ((31, 4, 64, 512), (32, 64, 784, 512), (32, 64, 1025, 512), (64, 64, 1025, 512),
+                                (64, 600, 784, 256), (64, 600, 784, 257), (64, 2000, 64, 512))] == \
+        [False, True, False, True, True, False, True]
