@@ -160,12 +160,18 @@ def _tmem_ksplit(num_tiles: int, tile_rows: int, num_chunks: int, B: int) -> int
 
 def _tmem_pays(sub_tiles: int, B: int) -> bool:
     """Whether the tensor-memory forms are offered for a BF16 contraction of so many (128 x 128)
-    sub-tiles: from about a 32-sample slice of one per SM. Below, their 128-sample slices leave SMs
-    idle, and timings of single eager launches (which the host bounds there) do not tell the forms
-    apart. Measured (us in a graph, best other form / best of these): 119 tiles, batch 32: 5.5 /
-    7.5, batch 64: 7.7 / 7.6; 60 tiles, batch 64: 5.4 / 6.9, batch 200: 11.3 / 7.8; 12 tiles, batch
-    200: 5.2 / 7.0, batch 512: 7.6 / 6.6. 16 forward steps of an HMM of 384 states, batch 200: 186 /
+    sub-tiles: from about a 32-sample slice of one per SM; for smaller batches, whose samples fill only a
+    part of the 128 lanes that every slice pays for, from more (0.4 of a full slice per SM up to 64
+    samples, one up to 32). Below, timings of single eager launches (which the host bounds there) do
+    not tell the forms apart. Measured (us in a graph, best other form / best of these, forward):
+    119 tiles, batch 32: 5.5 / 7.7, 64: 7.7 / 7.7, 200: 18.4 / 9.8; 480 tiles, batch 32: 13.3 / 18.9, 64: 22.9 /
+    19.7; 60 tiles, batch 64: 5.4 / 6.9, 200: 11.3 / 7.8; 12 tiles, batch 200: 5.2 / 7.0, 512: 7.6 / 6.6;
+    long tiles, 34 regions of 192 x 896, batch 32: 19.4 / 26.1, 48: 27.1 / 26.3; 10 of 288 x 960, batch 24:
+    10.0 / 14.2; 8 of 160 x 768, batch 48: 10.0 / 11.2; 60 of 128 x 512, batch 48: 16.1 / 12.7; 200 of 256 x
+    256, batch 24: 26.5 / 25.2, 32: 29.8 / 25.1. 16 forward steps of an HMM of 384 states, batch 200: 186 /
     203, 512: 221 / 206; of 512 states, batch 256: 190 / 193, 512: 274 / 234."""
+    if B <= 64:
+        return sub_tiles * B >= (128 if B <= 32 else 51) * _num_sms()
     return 8 * sub_tiles * -(-B // 32) >= 7 * _num_sms()
 
 

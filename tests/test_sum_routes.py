@@ -124,3 +124,13 @@ def test_ratio_workspace_is_no_larger_than_the_flows(ld, taken, calls, monkeypat
     layer.backward(buf, buf, buf, buf, torch.zeros([1]), None)
     assert ("pcb_flow_ratios" in calls) == taken
     assert [s for s in made if list(s)[-1] == ld] == ([[8 * 128, ld]] if taken else [])
+
+
+@pytest.mark.parametrize("sub_tiles,B,pays", [(480, 32, False), (800, 24, True), (476, 32, False), (119, 48, False), (240, 48, True),
+                                              (96, 48, False), (119, 64, True), (60, 64, False), (60, 200, True), (12, 200, False),
+                                              (12, 512, True)])
+def test_small_batches_keep_the_other_forms(sub_tiles, B, pays, monkeypatch):
+    """Slices of 128 samples are offered where they are filled, or there are many (the measured
+    cases beside the rule)."""
+    monkeypatch.setattr(mod, "_num_sms", lambda: 148)
+    assert mod._tmem_pays(sub_tiles, B) == pays
