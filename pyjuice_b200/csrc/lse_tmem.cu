@@ -754,6 +754,7 @@ lse_tmem_persistent_kernel(const float* __restrict__ src, const float* __restric
         put_rows();
         pcb::pdl_wait();
         if (S.nw == 2) copy_weights();
+        __syncwarp();
         tmem_alloc(slot, 512);
         fence_before_sync();
         taddr = columns();
